@@ -203,7 +203,7 @@ __global__ void __launch_bounds__(512) mcsub_kernel(const SubParams P) {
     const SpinDraws d = spin_draws<TT>(rng, need_roul, keys);
     float costheta;
     if (PHASE == kPhaseTT)
-      costheta = tt_sample<FAST>(P.phase, d.a, d.b);
+      costheta = tt_sample_param<FAST>(P.phase, d.a, d.b);
     else if (PHASE == kPhaseIsoRef)
       costheta = 2.f * d.a - 1.f;  // kernels.metal:252 overrides the HG sample
     else

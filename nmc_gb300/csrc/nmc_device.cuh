@@ -321,15 +321,19 @@ __device__ __forceinline__ void snell(float n1, float n2, float& ux, float& uy, 
 // HG (kernels.metal:696-703): cos = (d - (a / (b + c u))^2) * e with
 // a = 1-g^2, b = 1-g, c = 2g, d = 1+g^2, e = 1/(2g); mode 1 = isotropic
 // (g == 0), mode 2 = straight ahead (g == 1).
-// Two-term (kernels.metal:1060-1070): per branch q1/(2g), 1/q2, 1/q3,
-// -1/alpha, 1/(2g); iso flag when g == 0.
+// Two-term (kernels.metal:1060-1070): per lobe q1/(2g), 1/q2, 1/q3,
+// -1/alpha, 1/(2g); iso flag when g == 0.  A lobe is two aligned vector loads
+// from a table, a one-term draw two as well.
+struct __align__(16) PhaseLobe {
+  float q1e, iq2, iq3, ninva, e;
+  int iso, pad[2];
+};
 struct __align__(16) PhaseConst {
   float hg_a, hg_b, hg_c, hg_d, hg_e;
   int hg_mode;
   float cc;
-  float f_q1e, f_iq2, f_iq3, f_ninva, f_e;
-  float b_q1e, b_iq2, b_iq3, b_ninva, b_e;
-  int f_iso, b_iso;
+  int pad;
+  PhaseLobe f, b;
 };
 
 // Arithmetic of the photon step in two accuracy grades.  PRECISE uses
@@ -369,61 +373,87 @@ __device__ __forceinline__ float hg_sample(const PhaseConst& p, float u) {
   return p.hg_mode == 1 ? 2.f * u - 1.f : (p.hg_mode == 2 ? 1.f : c);
 }
 
-// Two-term sample from the branch choice and the sample uniform.
+// Two-term sample from the lobe choice and the sample uniform.  The lobe's
+// constants are selected and the power is taken once, so the lanes of a warp
+// that chose different lobes stay together (the isotropic form selects over
+// the general one, which may be NaN there).
 template <bool FAST>
-__device__ __forceinline__ float tt_sample(const PhaseConst& p, float uc, float u) {
-  float c;
-  if (uc <= p.cc) {
-    c = p.f_iso ? 2.f * u - 1.f
-                : p.f_q1e - Math<FAST>::pow(fmaf(u, p.f_iq2, (1.f - u) * p.f_iq3), p.f_ninva) * p.f_e;
-  } else {
-    c = p.b_iso ? 2.f * u - 1.f
-                : p.b_q1e - Math<FAST>::pow(fmaf(u, p.b_iq2, (1.f - u) * p.b_iq3), p.b_ninva) * p.b_e;
-    c = -c;
-  }
+__device__ __forceinline__ float lobe_sample(float q1e, float iq2, float iq3, float ninva, float e, int iso, bool fw,
+                                             float u) {
+  float c = q1e - Math<FAST>::pow(fmaf(u, iq2, (1.f - u) * iq3), ninva) * e;
+  c = iso ? 2.f * u - 1.f : c;
+  c = fw ? c : -c;
   if (c >= 1.f) c = 1.0f - 1e-9f;
   if (c <= -1.f) c = -(1.0f - 1e-9f);
   return c;
+}
+// p in shared or global memory: the lobe's address is selected
+template <bool FAST>
+__device__ __forceinline__ float tt_sample(const PhaseConst& p, float uc, float u) {
+  const bool fw = uc <= p.cc;
+  const PhaseLobe& q = fw ? p.f : p.b;
+  return lobe_sample<FAST>(q.q1e, q.iq2, q.iq3, q.ninva, q.e, q.iso, fw, u);
+}
+// p in the kernel's parameters: its constants are selected one by one
+template <bool FAST>
+__device__ __forceinline__ float tt_sample_param(const PhaseConst& p, float uc, float u) {
+  const bool fw = uc <= p.cc;
+  return lobe_sample<FAST>(fw ? p.f.q1e : p.b.q1e, fw ? p.f.iq2 : p.b.iq2, fw ? p.f.iq3 : p.b.iq3,
+                           fw ? p.f.ninva : p.b.ninva, fw ? p.f.e : p.b.e, fw ? p.f.iso : p.b.iso, fw, u);
 }
 
 // SPIN (kernels.metal:253-279, :704-730): rotate (ux, uy, uz) by polar
 // cos(theta) and azimuth psi = 2 pi u.  Near |uz| -> 1 the rotation and a
 // renormalisation run in FP64 (1 - uz^2 loses all FP32 bits there).
+//
+// spin_try is the common path without a branch; where it returns true the
+// direction is near vertical and its result is to be replaced by
+// spin_vertical's (from the old direction).  Kernels put that behind the one
+// test that their step's other rare events share.
+struct SpinTrig {
+  float sintheta, sinpsi, cospsi;
+};
 template <bool FAST>
-__device__ __forceinline__ void spin(float costheta, float upsi, float& ux, float& uy,
-                                     float& uz) {
-  const float sintheta = Math<FAST>::sqrt(fmaxf(fmaf(-costheta, costheta, 1.f), 0.f));
-  float sinpsi, cospsi;
-  Math<FAST>::sincos2pi(upsi, &sinpsi, &cospsi);
+__device__ __forceinline__ bool spin_try(float costheta, float upsi, float ux, float uy, float uz, SpinTrig& t,
+                                         float& nx, float& ny, float& nz) {
+  t.sintheta = Math<FAST>::sqrt(fmaxf(fmaf(-costheta, costheta, 1.f), 0.f));
+  Math<FAST>::sincos2pi(upsi, &t.sinpsi, &t.cospsi);
+  const float temp2 = fmaf(-uz, uz, 1.f);
+  const float itemp = rsqrtf(temp2);
+  const float temp = temp2 * itemp;
+  nx = fmaf(t.sintheta * (ux * uz * t.cospsi - uy * t.sinpsi), itemp, ux * costheta);
+  ny = fmaf(t.sintheta * (uy * uz * t.cospsi + ux * t.sinpsi), itemp, uy * costheta);
+  nz = fmaf(-t.sintheta * t.cospsi, temp, uz * costheta);
+  return 1.f - fabsf(uz) < 1e-5f;
+}
+__device__ __forceinline__ void spin_vertical(float costheta, const SpinTrig& t, float ux, float uy, float uz,
+                                              float& nx, float& ny, float& nz) {
   const float auz = fabsf(uz);
-  // one test on the common path; the two near-vertical cases behind it
-  if (__builtin_expect(1.f - auz < 1e-5f, 0)) {
-    if (auz >= 1.f) {  // 1 - |uz| <= 1e-12 in FP32
-      ux = sintheta * cospsi;
-      uy = sintheta * sinpsi;
-      uz = uz >= 0.f ? costheta : -costheta;
-    } else {
-      const double dz = uz, temp = sqrt(1.0 - dz * dz);
-      const double st = sintheta, ct = costheta, cp = cospsi, sp = sinpsi;
-      double nx = st * (ux * dz * cp - uy * sp) / temp + ux * ct;
-      double ny = st * (uy * dz * cp + ux * sp) / temp + uy * ct;
-      double nz = -st * cp * temp + dz * ct;
-      const double inv = 1.0 / sqrt(nx * nx + ny * ny + nz * nz);
-      ux = (float)(nx * inv);
-      uy = (float)(ny * inv);
-      uz = (float)(nz * inv);
-    }
+  if (auz >= 1.f) {  // 1 - |uz| <= 1e-12 in FP32
+    nx = t.sintheta * t.cospsi;
+    ny = t.sintheta * t.sinpsi;
+    nz = uz >= 0.f ? costheta : -costheta;
   } else {
-    const float temp2 = fmaf(-uz, uz, 1.f);
-    const float itemp = rsqrtf(temp2);
-    const float temp = temp2 * itemp;
-    const float nx = fmaf(sintheta * (ux * uz * cospsi - uy * sinpsi), itemp, ux * costheta);
-    const float ny = fmaf(sintheta * (uy * uz * cospsi + ux * sinpsi), itemp, uy * costheta);
-    const float nz = fmaf(-sintheta * cospsi, temp, uz * costheta);
-    ux = nx;
-    uy = ny;
-    uz = nz;
+    const double dz = uz, temp = sqrt(1.0 - dz * dz);
+    const double st = t.sintheta, ct = costheta, cp = t.cospsi, sp = t.sinpsi;
+    const double x = st * (ux * dz * cp - uy * sp) / temp + ux * ct;
+    const double y = st * (uy * dz * cp + ux * sp) / temp + uy * ct;
+    const double z = -st * cp * temp + dz * ct;
+    const double inv = 1.0 / sqrt(x * x + y * y + z * z);
+    nx = (float)(x * inv);
+    ny = (float)(y * inv);
+    nz = (float)(z * inv);
   }
+}
+template <bool FAST>
+__device__ __forceinline__ void spin(float costheta, float upsi, float& ux, float& uy, float& uz) {
+  SpinTrig t;
+  float nx, ny, nz;
+  if (__builtin_expect(spin_try<FAST>(costheta, upsi, ux, uy, uz, t, nx, ny, nz), 0))
+    spin_vertical(costheta, t, ux, uy, uz, nx, ny, nz);
+  ux = nx;
+  uy = ny;
+  uz = nz;
 }
 
 // ----------------------------------------------------------- index checks

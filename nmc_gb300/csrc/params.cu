@@ -62,21 +62,21 @@ PhaseConst phase_const(const nmc_tissue_params& tp, int t) {
   }
   const double gf = tp.gf[t], af = tp.af[t], gb = tp.gb[t], ab = tp.ab[t];  // :894-905
   p.cc = tp.CC[t];
-  p.f_iso = gf == 0.0;
-  p.b_iso = gb == 0.0;
-  if (!p.f_iso) {
-    p.f_q1e = (float)((1.0 + gf * gf) / (2.0 * gf));
-    p.f_iq2 = (float)(1.0 / std::pow(1.0 - gf, 2.0 * af));
-    p.f_iq3 = (float)(1.0 / std::pow(1.0 + gf, 2.0 * af));
-    p.f_ninva = (float)(-1.0 / af);
-    p.f_e = (float)(1.0 / (2.0 * gf));
+  p.f.iso = gf == 0.0;
+  p.b.iso = gb == 0.0;
+  if (!p.f.iso) {
+    p.f.q1e = (float)((1.0 + gf * gf) / (2.0 * gf));
+    p.f.iq2 = (float)(1.0 / std::pow(1.0 - gf, 2.0 * af));
+    p.f.iq3 = (float)(1.0 / std::pow(1.0 + gf, 2.0 * af));
+    p.f.ninva = (float)(-1.0 / af);
+    p.f.e = (float)(1.0 / (2.0 * gf));
   }
-  if (!p.b_iso) {
-    p.b_q1e = (float)((1.0 + gb * gb) / (2.0 * gb));
-    p.b_iq2 = (float)(1.0 / std::pow(1.0 - gb, 2.0 * ab));
-    p.b_iq3 = (float)(1.0 / std::pow(1.0 + gb, 2.0 * ab));
-    p.b_ninva = (float)(-1.0 / ab);
-    p.b_e = (float)(1.0 / (2.0 * gb));
+  if (!p.b.iso) {
+    p.b.q1e = (float)((1.0 + gb * gb) / (2.0 * gb));
+    p.b.iq2 = (float)(1.0 / std::pow(1.0 - gb, 2.0 * ab));
+    p.b.iq3 = (float)(1.0 / std::pow(1.0 + gb, 2.0 * ab));
+    p.b.ninva = (float)(-1.0 / ab);
+    p.b.e = (float)(1.0 / (2.0 * gb));
   }
   return p;
 }

@@ -15,6 +15,15 @@
 // Per-set totals are u64 fixed point in shared memory, folded into global
 // memory once per block; the escaping flux J(r) of each set goes straight to
 // global u64 atomics (one deposit per escaping photon).
+//
+// A photon keeps its set's constants in registers.  Read from the table at
+// every hop, the lanes of a warp (in different sets) took up to 32 L1 lines
+// per load and waited 3.4 cycles per instruction for them.  The kernel needs
+// 74-79 registers for it and runs 3 blocks of 256 per SM: 351 two-term sets
+// of 1.4e7 photons in 71.0 ms, against 92.3 ms with the table reads at 4
+// blocks (and 85.6 ms with the constants in registers squeezed to 4 blocks);
+// 3.5e6 photons, where fewer resident photons also shorten the tail, 37.6
+// against 53.8 ms.
 #include <cuda_runtime.h>
 
 #include "engine.h"
@@ -23,7 +32,7 @@ namespace nmc {
 namespace {
 
 template <int PHASE, bool FAST>
-__global__ void __launch_bounds__(256) sweep_kernel(const SweepParams P) {
+__global__ void __launch_bounds__(256, 3) sweep_kernel(const SweepParams P) {
   using M = Math<FAST>;
   constexpr bool TT = PHASE == kPhaseTT;
   extern __shared__ unsigned long long s_sum[];  // nsets x 5: photons, hops, S, A, E
@@ -36,6 +45,9 @@ __global__ void __launch_bounds__(256) sweep_kernel(const SweepParams P) {
   PhiloxRng<TT> rng;
   float x = 0.f, y = 0.f, z = 0.f, ux = 0.f, uy = 0.f, uz = 1.f, W = 0.f, step_u = 1.f;
   float rsp = 0.f, Atot = 0.f, E = 0.f;
+  // the set's mu_t, 1 - albedo and phase constants, kept over the photon's life
+  float mut = 1.f, oma = 0.f;
+  PhaseConst ph;
   uint32_t nsc = 0, nsub = 0, k1 = P.k1;
   int set = 0;
   const SweepSetDev* S = P.sets;
@@ -99,13 +111,15 @@ __global__ void __launch_bounds__(256) sweep_kernel(const SweepParams P) {
         uz = costheta;
       }
       step_u = rng.first_step(k0, k1);
+      mut = __ldg(&S->mut);
+      oma = 1.f - __ldg(&S->albedo);
+      ph = S->ph;
       W = 1.f - rsp;
       Atot = E = 0.f;
       nsc = nsub = 0;
       alive = true;
     }
 
-    const float mut = __ldg(&S->mut);
     // ---- HOP (:183-187)
     const float s = M::div(M::neglog(step_u), mut);
     x = fmaf(s, ux, x);
@@ -133,7 +147,7 @@ __global__ void __launch_bounds__(256) sweep_kernel(const SweepParams P) {
       uz = -uz;
     }
     // ---- DROP (:224-234): absorbed weight only (no F(r,z) in sweeps)
-    const float absorb = W * (1.f - __ldg(&S->albedo));
+    const float absorb = W * oma;
     W -= absorb;
     Atot += absorb;
     // ---- SPIN (:243-279), ROULETTE (:289-294), next HOP's draw
@@ -141,19 +155,27 @@ __global__ void __launch_bounds__(256) sweep_kernel(const SweepParams P) {
     const SpinDraws dr = rng.spin_draws(need_roul, k0, k1);
     float costheta;
     if (PHASE == kPhaseTT)
-      costheta = tt_sample<FAST>(S->ph, dr.a, dr.b);
+      costheta = tt_sample_param<FAST>(ph, dr.a, dr.b);
     else if (PHASE == kPhaseIsoRef)
       costheta = 2.f * dr.a - 1.f;
     else
-      costheta = hg_sample<FAST>(S->ph, dr.a);
-    spin<FAST>(costheta, TT ? dr.c : dr.b, ux, uy, uz);
+      costheta = hg_sample<FAST>(ph, dr.a);
+    SpinTrig trig;
+    float nx, ny, nz;
+    const bool vertical = spin_try<FAST>(costheta, TT ? dr.c : dr.b, ux, uy, uz, trig, nx, ny, nz);
     ++nsc;
-    if (need_roul) {
-      if (dr.roul <= kCHANCE)
-        W /= kCHANCE;
-      else
-        alive = false;
+    if (__builtin_expect(vertical | need_roul, 0)) {
+      if (vertical) spin_vertical(costheta, trig, ux, uy, uz, nx, ny, nz);
+      if (need_roul) {
+        if (dr.roul <= kCHANCE)
+          W /= kCHANCE;
+        else
+          alive = false;
+      }
     }
+    ux = nx;
+    uy = ny;
+    uz = nz;
     step_u = dr.step;
     if (alive && nsub >= P.step_cap) {
       alive = false;
