@@ -39,6 +39,18 @@
 //   d score/d mua_l = -score L_l,
 //   d score/d mus_l = score (n_l / mus_l - L_l),
 //   d score/d g_l   = score Q_l.
+//
+// One trip of a lane is one interaction, with the boundary it may cross on the
+// way; a lane whose photon ended takes the next one.  The kernel is bound by
+// instruction issue (76% of the slots), so the trip avoids work that most
+// lanes do not need: it divides for the distance to the boundary only near it,
+// draws the Fresnel choice only where the reflectance is between 0 and 1,
+// puts the rare events (a near-vertical direction, a new layer, the roulette,
+// a carry of the A(z) sum) behind one test, and goes on to the interaction
+// after a crossing.  Three-layer skin, 4e6 photons of 1520 interactions:
+// 69.4 -> 53.6 ms, 10.3 -> 8.0 warp instructions per interaction at 21.0 ->
+// 22.9 active lanes (1e6 photons: 26.9 -> 21 ms, 10 ms of it the longest
+// photon).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -94,7 +106,7 @@ struct LayParams {
 };
 
 template <bool FAST, bool ADJ, bool REF>
-__global__ void __launch_bounds__(256) layered_kernel(const LayParams P) {
+__global__ void __launch_bounds__(256, 4) layered_kernel(const LayParams P) {
   using M = Math<FAST>;
   __shared__ LayDev s_lay[kMaxLayers];
   __shared__ double s_sum[NMC_LAY_FIELDS];
@@ -112,37 +124,75 @@ __global__ void __launch_bounds__(256) layered_kernel(const LayParams P) {
   if (ADJ)
     for (int i = threadIdx.x; i < 3 * kMaxAdjLayers; i += blockDim.x) s_grad[i] = 0.0;
   __syncthreads();
+
+  float x = 0.f, y = 0.f, z = 0.f, ux = 0.f, uy = 0.f, uz = 1.f, w = 0.f, sleft = 0.f;
+  int L = 0;
+  uint32_t c0 = 0, c1 = 0, hop = 0, ev = 0;
+  bool alive = false, have = false;
+  float rd = 0.f, tt = 0.f;
+  int dep_l = 0;        // the layer whose absorbed weight dep_w holds
+  float dep_w = 0.f;    // merged while the photon stays in one layer
+  float aL[ADJ ? kMaxAdjLayers : 1], aN[ADJ ? kMaxAdjLayers : 1], aQ[ADJ ? kMaxAdjLayers : 1];
+  float score = 0.f;
+  TausRng tr;
+  uint4 r = make_uint4(0u, 0u, 0u, 0u);  // Philox block of the coming interaction
+
+  // path length of the rest of the step in layer L, and to the boundary ahead
+  auto path = [&]() { return s_lay[L].inv_mut > 0.f ? sleft * s_lay[L].inv_mut : INFINITY; };
+  auto ahead = [&]() {
+    return uz > 0.f ? (s_lay[L].z1 - z) / uz : (uz < 0.f ? (s_lay[L].z0 - z) / uz : INFINITY);
+  };
+
   while (true) {
-    const unsigned long long g = next_photon(P.work);
-    if (g >= P.n) break;
-    const unsigned long long pid = P.first + g;
-    const uint32_t c0 = (uint32_t)pid, c1 = (uint32_t)(pid >> 32);
-    float x = 0.f, y = 0.f, z = 0.f, ux = 0.f, uy = 0.f, uz = 1.f, w = P.w0, sleft = 0.f;
-    int L = 0;
-    uint32_t hop = 0, ev = 0;
-    bool alive = true;
-    float rd = 0.f, tt = 0.f;
-    int dep_l = 0;        // the layer whose absorbed weight dep_w holds
-    float dep_w = 0.f;    // merged while the photon stays in one layer
-    float aL[ADJ ? kMaxAdjLayers : 1], aN[ADJ ? kMaxAdjLayers : 1], aQ[ADJ ? kMaxAdjLayers : 1];
-    float score = 0.f;
-    if (ADJ)
-      for (int l = 0; l < P.nl; ++l) aL[l] = aN[l] = aQ[l] = 0.f;
-    TausRng tr;
-    uint4 r = make_uint4(0u, 0u, 0u, 0u);
-    if (REF) {
-      tr.init_photon(pid, P.batch, false, false);
-      tr.next();  // the launch draw (radius 0: the beam stays on the axis)
-    } else {
-      r = philox4x32_10(make_uint4(c0, c1, 0u, kLayTag), RoundKeys{P.rk});
+    if (!alive) {
+      if (have) {
+        if (dep_w > 0.f && idx_ok(dep_l, (unsigned)P.nl, P.flags)) atomicAdd(s_al + dep_l, to_fix(dep_w));
+        atomicAdd(&s_sum[NMC_LAY_PHOTONS], 1.0);
+        atomicAdd(&s_sum[NMC_LAY_RD], (double)rd);
+        atomicAdd(&s_sum[NMC_LAY_RD2], (double)rd * (double)rd);
+        atomicAdd(&s_sum[NMC_LAY_TT], (double)tt);
+        atomicAdd(&s_sum[NMC_LAY_TT2], (double)tt * (double)tt);
+        atomicAdd(&s_sum[NMC_LAY_INTERACTIONS], (double)hop);
+        if (ADJ && score != 0.f)
+          for (int l = 0; l < P.nl; ++l) {
+            atomicAdd(&s_grad[l], (double)(-score * aL[l]));
+            atomicAdd(&s_grad[kMaxAdjLayers + l],
+                      (double)(score * (s_lay[l].mus > 0.f ? aN[l] / s_lay[l].mus - aL[l] : -aL[l])));
+            atomicAdd(&s_grad[2 * kMaxAdjLayers + l], (double)(score * aQ[l]));
+          }
+      }
+      const unsigned long long g = next_photon(P.work);
+      if (g >= P.n) break;
+      have = true;
+      alive = true;
+      const unsigned long long pid = P.first + g;
+      c0 = (uint32_t)pid, c1 = (uint32_t)(pid >> 32);
+      x = y = z = ux = uy = 0.f;
+      uz = 1.f;
+      w = P.w0;
+      L = dep_l = 0;
+      hop = ev = 0;
+      rd = tt = dep_w = score = 0.f;
+      if (ADJ)
+        for (int l = 0; l < P.nl; ++l) aL[l] = aN[l] = aQ[l] = 0.f;
+      if (REF) {
+        tr.init_photon(pid, P.batch, false, false);
+        tr.next();  // the launch draw (radius 0: the beam stays on the axis)
+      } else {
+        r = philox4x32_10(make_uint4(c0, c1, 0u, kLayTag), RoundKeys{P.rk});
+      }
+      sleft = M::neglog(REF ? tr.step_draw() : u01(r.x));
     }
-    while (alive) {
-      const LayDev& Ly = s_lay[L];
-      if (sleft <= 0.f) sleft = M::neglog(REF ? tr.step_draw() : u01(r.x));
-      // distance to the layer boundary ahead
-      const float db = uz > 0.f ? (Ly.z1 - z) / uz : (uz < 0.f ? (Ly.z0 - z) / uz : INFINITY);
-      const float s = Ly.inv_mut > 0.f ? sleft * Ly.inv_mut : INFINITY;
+
+    float s = path();
+    // A step reaches the boundary when s >= distance / uz.  Most do not come
+    // near it, which a product shows: only the others divide.  (The product
+    // and the quotient are within 2^-22 of the exact values.)
+    const float dz = uz > 0.f ? s_lay[L].z1 - z : z - s_lay[L].z0;
+    if (!(s * fabsf(uz) * 1.000001f < dz)) {
+      const float db = ahead();
       if (s >= db) {  // reaches the boundary: CROSS
+        const LayDev& Ly = s_lay[L];
         x = fmaf(db, ux, x);
         y = fmaf(db, uy, y);
         z = uz > 0.f ? Ly.z1 : Ly.z0;
@@ -153,11 +203,15 @@ __global__ void __launch_bounds__(256) layered_kernel(const LayParams P) {
         const float nt = Ln < 0 ? P.n_above : (Ln >= P.nl ? P.n_below : s_lay[Ln].n);
         float uzt = 0.f;
         const float R = rfresnel(Ly.n, nt, fabsf(uz), &uzt);
-        const float uf =
-            REF ? tr.next() : u01(philox4x32_10(make_uint4(c0, c1, ev | 0x80000000u, kLayTag), RoundKeys{P.rk}).x);
+        // a draw lies in (0, 1): matched layers and total reflection need none
+        bool reflect = R >= 1.f;
+        if (REF)
+          reflect = tr.next() <= R;
+        else if (R > 0.f && R < 1.f)
+          reflect = u01(philox4x32_10(make_uint4(c0, c1, ev | 0x80000000u, kLayTag), RoundKeys{P.rk}).x) <= R;
         ++ev;
-        if (uf <= R) {
-          uz = -uz;  // reflected
+        if (reflect) {
+          uz = -uz;
         } else if (Ln < 0 || Ln >= P.nl) {  // escapes
           const float rr = sqrtf(x * x + y * y);
           const int ir = min((int)(rr * P.idr), P.nr);
@@ -182,66 +236,78 @@ __global__ void __launch_bounds__(256) layered_kernel(const LayParams P) {
           atomicOr(P.flags, (unsigned int)NMC_DEVFLAG_STEPCAP);
           alive = false;
         }
-        continue;
+        if (alive) {  // go on from the boundary: most steps now end inside the layer
+          if (sleft <= 0.f) sleft = M::neglog(REF ? tr.step_draw() : u01(r.x));
+          s = path();
+        }
+        if (!alive || s >= ahead()) continue;
       }
-      // interaction inside the layer: HOP, DROP, SPIN, ROULETTE
-      x = fmaf(s, ux, x);
-      y = fmaf(s, uy, y);
-      z = fmaf(s, uz, z);
-      sleft = 0.f;
-      if (ADJ) {
-        aL[L] += s;
-        aN[L] += 1.f;
+    }
+    // interaction inside the layer: HOP, DROP, SPIN, ROULETTE
+    const LayDev& Ly = s_lay[L];
+    x = fmaf(s, ux, x);
+    y = fmaf(s, uy, y);
+    z = fmaf(s, uz, z);
+    if (ADJ) {
+      aL[L] += s;
+      aN[L] += 1.f;
+    }
+    const float absorb = w * Ly.mua * Ly.inv_mut;
+    w -= absorb;
+    int iz = 0;
+    unsigned int dep = 0u, old = 0u;  // the deposit and the low word it met
+    if (absorb > 0.f) {
+      iz = min(max((int)(z * P.idz), 0), P.nz);
+      if (idx_ok(iz, (unsigned)P.nz + 1u, P.flags)) {
+        if (P.smem_az) {
+          // below 1 the fixed-point deposit fits the low word; its carry is rare
+          dep = __float2uint_rn(absorb * kFix);
+          old = atomicAdd(reinterpret_cast<unsigned int*>(s_az + iz), dep);
+        } else {
+          atomicAdd(P.a_z + iz, to_fix(absorb));
+        }
       }
-      const float absorb = w * Ly.mua * Ly.inv_mut;
-      w -= absorb;
-      if (absorb > 0.f) {
+      if (P.a_rz) {
         const unsigned long long fa = to_fix(absorb);
-        const int iz = min(max((int)(z * P.idz), 0), P.nz);
-        if (idx_ok(iz, (unsigned)P.nz + 1u, P.flags)) atomicAdd((P.smem_az ? s_az : P.a_z) + iz, fa);
-        if (L != dep_l) {
-          if (dep_w > 0.f && idx_ok(dep_l, (unsigned)P.nl, P.flags)) atomicAdd(s_al + dep_l, to_fix(dep_w));
-          dep_l = L;
-          dep_w = 0.f;
-        }
-        dep_w += absorb;
-        if (P.a_rz) {
-          const int ir = min((int)(sqrtf(x * x + y * y) * P.idr), P.nr);
-          if (idx_ok((size_t)ir * (P.nz + 1) + iz, (size_t)(P.nr + 1) * (P.nz + 1), P.flags))
-            atomicAdd(P.a_rz + (size_t)ir * (P.nz + 1) + iz, fa);
-        }
+        const int ir = min((int)(sqrtf(x * x + y * y) * P.idr), P.nr);
+        if (idx_ok((size_t)ir * (P.nz + 1) + iz, (size_t)(P.nr + 1) * (P.nz + 1), P.flags))
+          atomicAdd(P.a_rz + (size_t)ir * (P.nz + 1) + iz, fa);
       }
-      const float ucos = REF ? tr.next() : u01(r.y);
-      const float cth = P.iso ? 2.f * ucos - 1.f : hg_sample<FAST>(Ly.ph, ucos);
-      if (ADJ && Ly.ph.hg_mode == 0) aQ[L] += dln_hg_dg(Ly.g, cth);
-      spin<FAST>(cth, REF ? tr.next() : u01(r.z), ux, uy, uz);
+    }
+    const float ucos = REF ? tr.next() : u01(r.y);
+    const float cth = P.iso ? 2.f * ucos - 1.f : hg_sample<FAST>(Ly.ph, ucos);
+    if (ADJ && Ly.ph.hg_mode == 0) aQ[L] += dln_hg_dg(Ly.g, cth);
+    SpinTrig trig;
+    float nx, ny, nz;
+    const bool vertical = spin_try<FAST>(cth, REF ? tr.next() : u01(r.z), ux, uy, uz, trig, nx, ny, nz);
+    ++hop;
+    // the rare events of an interaction behind one test
+    const bool other = L != dep_l, carry = old + dep < old;
+    if (__builtin_expect(vertical | other | carry | (w < kTHRESHOLD) | (hop > P.step_cap), 0)) {
+      if (carry) atomicAdd(reinterpret_cast<unsigned int*>(s_az + iz) + 1, 1u);
+      if (vertical) spin_vertical(cth, trig, ux, uy, uz, nx, ny, nz);
+      if (other && absorb > 0.f) {
+        if (dep_w > 0.f && idx_ok(dep_l, (unsigned)P.nl, P.flags)) atomicAdd(s_al + dep_l, to_fix(dep_w));
+        dep_l = L;
+        dep_w = 0.f;
+      }
       if (w < kTHRESHOLD) {
         if ((REF ? tr.next() : u01(r.w)) <= kCHANCE)
           w /= kCHANCE;
         else
           alive = false;
       }
-      ++hop;
       if (hop > P.step_cap) {
         atomicOr(P.flags, (unsigned int)NMC_DEVFLAG_STEPCAP);
         alive = false;
       }
-      if (!REF) r = philox4x32_10(make_uint4(c0, c1, hop, kLayTag), RoundKeys{P.rk});
     }
-    if (dep_w > 0.f && idx_ok(dep_l, (unsigned)P.nl, P.flags)) atomicAdd(s_al + dep_l, to_fix(dep_w));
-    atomicAdd(&s_sum[NMC_LAY_PHOTONS], 1.0);
-    atomicAdd(&s_sum[NMC_LAY_RD], (double)rd);
-    atomicAdd(&s_sum[NMC_LAY_RD2], (double)rd * (double)rd);
-    atomicAdd(&s_sum[NMC_LAY_TT], (double)tt);
-    atomicAdd(&s_sum[NMC_LAY_TT2], (double)tt * (double)tt);
-    atomicAdd(&s_sum[NMC_LAY_INTERACTIONS], (double)hop);
-    if (ADJ && score != 0.f)
-      for (int l = 0; l < P.nl; ++l) {
-        atomicAdd(&s_grad[l], (double)(-score * aL[l]));
-        atomicAdd(&s_grad[kMaxAdjLayers + l],
-                  (double)(score * (s_lay[l].mus > 0.f ? aN[l] / s_lay[l].mus - aL[l] : -aL[l])));
-        atomicAdd(&s_grad[2 * kMaxAdjLayers + l], (double)(score * aQ[l]));
-      }
+    dep_w += absorb;
+    ux = nx;
+    uy = ny;
+    uz = nz;
+    if (!REF) r = philox4x32_10(make_uint4(c0, c1, hop, kLayTag), RoundKeys{P.rk});
+    if (!REF || alive) sleft = M::neglog(REF ? tr.step_draw() : u01(r.x));
   }
   __syncthreads();
   for (int i = threadIdx.x; i < n_priv; i += blockDim.x) {
@@ -383,7 +449,10 @@ nmc_status layered_impl(int32_t device, const nmc_layered_config* cfg, const nmc
       : ref ? (fast ? (const void*)layered_kernel<true, false, true> : (const void*)layered_kernel<false, false, true>)
             : (fast ? (const void*)layered_kernel<true, false, false> : (const void*)layered_kernel<false, false, false>);
   // A(z) joins the per-layer sums in shared memory while both fit in 16 KB
-  P.smem_az = (size_t)(c.n_layers + nz1) * 8 <= 16384 ? 1 : 0;
+  // and every deposit is below 1 (no pure absorber under a whole weight)
+  float most = 0.f;
+  for (const LayDev& d : lay) most = std::max(most, P.w0 * d.mua * d.inv_mut);
+  P.smem_az = (size_t)(c.n_layers + nz1) * 8 <= 16384 && most < 1.f ? 1 : 0;
   const size_t smem = (size_t)(c.n_layers + (P.smem_az ? nz1 : 0)) * 8;
   int per_sm = 0, nsm = 0;
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device);
