@@ -208,16 +208,24 @@ __global__ void __launch_bounds__(512) mcsub_kernel(const SubParams P) {
       costheta = 2.f * d.a - 1.f;  // kernels.metal:252 overrides the HG sample
     else
       costheta = hg_sample<FAST>(P.phase, d.a);
-    spin<FAST>(costheta, TT ? d.c : d.b, ux, uy, uz);
+    SpinTrig trig;
+    float nx, ny, nz;
+    const bool vertical = spin_try<FAST>(costheta, TT ? d.c : d.b, ux, uy, uz, trig, nx, ny, nz);
     ++nsc;
-    if (need_roul) {
-      if (d.roul <= kCHANCE) {
-        W /= kCHANCE;
-      } else {
-        if (TRACE) fate = NMC_FATE_ROULETTE;
-        alive = false;
+    if (__builtin_expect(vertical | need_roul, 0)) {
+      if (vertical) spin_vertical(costheta, trig, ux, uy, uz, nx, ny, nz);
+      if (need_roul) {
+        if (d.roul <= kCHANCE) {
+          W /= kCHANCE;
+        } else {
+          if (TRACE) fate = NMC_FATE_ROULETTE;
+          alive = false;
+        }
       }
     }
+    ux = nx;
+    uy = ny;
+    uz = nz;
     if (TRACE && nev < P.trace.k_events) {
       P.trace.events[pidx * P.trace.k_events + nev] = make_float4(x, y, z, W);
       ++nev;

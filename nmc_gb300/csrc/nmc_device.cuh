@@ -408,7 +408,7 @@ __device__ __forceinline__ float tt_sample_param(const PhaseConst& p, float uc, 
 //
 // spin_try is the common path without a branch; where it returns true the
 // direction is near vertical and its result is to be replaced by
-// spin_vertical's (from the old direction).  Kernels put that behind the one
+// spin_vertical's (from the old direction).  The kernels put that behind the one
 // test that their step's other rare events share.
 struct SpinTrig {
   float sintheta, sinpsi, cospsi;
@@ -445,17 +445,6 @@ __device__ __forceinline__ void spin_vertical(float costheta, const SpinTrig& t,
     nz = (float)(z * inv);
   }
 }
-template <bool FAST>
-__device__ __forceinline__ void spin(float costheta, float upsi, float& ux, float& uy, float& uz) {
-  SpinTrig t;
-  float nx, ny, nz;
-  if (__builtin_expect(spin_try<FAST>(costheta, upsi, ux, uy, uz, t, nx, ny, nz), 0))
-    spin_vertical(costheta, t, ux, uy, uz, nx, ny, nz);
-  ux = nx;
-  uy = ny;
-  uz = nz;
-}
-
 // ----------------------------------------------------------- index checks
 // The checked build (-DNMC_CHECK_BOUNDS, nmc_gb300/_build/checked/) tests
 // every tally index against its buffer; an index out of range raises
