@@ -37,6 +37,16 @@ struct AdjEvent {
   float pad;
 };
 
+// The latency variant of a kernel runs few photons per lane: kLatBlocks blocks
+// of kLatBlock threads per SM (4 warps per scheduler, up to 128 registers)
+// instead of a full SM, and, when the queue is empty, warps that "go on thin":
+// once at most kThinPhotons of a warp's lanes have a photon, the others
+// compute the random part of the coming hops, which depends on the photon and
+// the hop's number alone.  A photon looks for that every kThinLook scatterings.
+constexpr int kLatBlock = 256, kLatBlocks = 2;
+constexpr int kThinPhotons = 8;
+constexpr unsigned int kThinLook = 16;
+
 // Voxel kernels (MCXYZKernel kernels.metal:321-754 and MCXYZKernelTT
 // :757-1118).  Photon positions are kept as an integer voxel-lattice cell
 // (k = floor(x / d), unbounded) plus an FP32 offset inside the cell.
@@ -131,6 +141,7 @@ struct SubParams {
   int skip_F;        // no F(r,z) tally
   int global_tallies;  // F(r,z), J(r) straight to global memory (no shared-memory privatisation)
   uint32_t per_fetch;  // photons a thread takes from the queue at a time (>= 1)
+  unsigned int lanes;  // > 0: the latency variant, with this many lanes of a warp taking photons
   unsigned long long* J;  // fixed point 2^-32, BINS+1
   unsigned long long* F;  // (BINS+1)^2
   DevSums* sums;

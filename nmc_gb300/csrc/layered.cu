@@ -277,9 +277,9 @@ __global__ void __launch_bounds__(256, 4) layered_kernel(const LayParams P) {
     const float ucos = REF ? tr.next() : u01(r.y);
     const float cth = P.iso ? 2.f * ucos - 1.f : hg_sample<FAST>(Ly.ph, ucos);
     if (ADJ && Ly.ph.hg_mode == 0) aQ[L] += dln_hg_dg(Ly.g, cth);
-    SpinTrig trig;
+    const SpinTrig trig = spin_trig<FAST>(cth, REF ? tr.next() : u01(r.z));
     float nx, ny, nz;
-    const bool vertical = spin_try<FAST>(cth, REF ? tr.next() : u01(r.z), ux, uy, uz, trig, nx, ny, nz);
+    const bool vertical = spin_try(cth, trig, ux, uy, uz, nx, ny, nz);
     ++hop;
     // the rare events of an interaction behind one test
     const bool other = L != dep_l, carry = old + dep < old;

@@ -669,9 +669,9 @@ __global__ void __launch_bounds__(256, 4) mcxyz_kernel(const XyzParams P) {
       const PhaseConst& ph = SW ? P.sw_phase[sbase + tiss] : s_ph[tiss];
       costheta = TT ? tt_sample<FAST>(ph, d.a, d.b) : hg_sample<FAST>(ph, d.a);
     }
-    SpinTrig trig;
+    const SpinTrig trig = spin_trig<FAST>(costheta, TT ? d.c : d.b);
     float nx, ny, nz;
-    const bool vertical = spin_try<FAST>(costheta, TT ? d.c : d.b, ux, uy, uz, trig, nx, ny, nz);
+    const bool vertical = spin_try(costheta, trig, ux, uy, uz, nx, ny, nz);
     ++nsc;
     // one test for the rare events of a hop's end: a near-vertical direction,
     // the roulette and both kills (W < MIN_VALUE implies W < THRESHOLD).  With

@@ -414,10 +414,14 @@ struct SpinTrig {
   float sintheta, sinpsi, cospsi;
 };
 template <bool FAST>
-__device__ __forceinline__ bool spin_try(float costheta, float upsi, float ux, float uy, float uz, SpinTrig& t,
-                                         float& nx, float& ny, float& nz) {
+__device__ __forceinline__ SpinTrig spin_trig(float costheta, float upsi) {
+  SpinTrig t;
   t.sintheta = Math<FAST>::sqrt(fmaxf(fmaf(-costheta, costheta, 1.f), 0.f));
   Math<FAST>::sincos2pi(upsi, &t.sinpsi, &t.cospsi);
+  return t;
+}
+__device__ __forceinline__ bool spin_try(float costheta, const SpinTrig& t, float ux, float uy, float uz, float& nx,
+                                         float& ny, float& nz) {
   const float temp2 = fmaf(-uz, uz, 1.f);
   const float itemp = rsqrtf(temp2);
   const float temp = temp2 * itemp;

@@ -423,11 +423,23 @@ nmc_status launch(nmc_handle* h, uint64_t first, uint64_t n, nmc_photon_record* 
     p.n = n;
     p.trace = tr;
     block = h->ext.block_size > 0 ? h->ext.block_size : 512;
+    // Up to four photons per lane of the latency variant it is the faster one
+    // (semi-infinite medium, mua 1, mus 100: 1e4 photons 0.58 against 0.90 ms,
+    // 1e5 1.01 / 1.58, 3e5 1.71 / 1.82, 1e6 4.44 / 3.82 ms); below one photon
+    // per lane they are spread over all its warps.
+    const uint64_t warps = (uint64_t)h->nsm * nmc::kLatBlocks * (nmc::kLatBlock / 32);
+    const uint64_t items = (n + p.per_fetch - 1) / p.per_fetch;
+    const bool lat = !trace && h->ext.block_size <= 0 && h->ext.blocks_per_sm <= 0 && items <= warps * 128;
+    if (lat) {
+      block = nmc::kLatBlock;
+      p.lanes = (unsigned int)std::min<uint64_t>(32, (items + warps - 1) / warps);
+    }
     NMC_CUDA(h, nmc::mcsub_occupancy(p, trace, block, &per_sm));
     if (h->ext.blocks_per_sm > 0) per_sm = std::min(per_sm, (int)h->ext.blocks_per_sm);
+    if (lat) per_sm = std::min(per_sm, nmc::kLatBlocks);
     if (per_sm < 1) return fail(h, NMC_EDEVICE, "mcsub kernel does not fit on an SM with this block size");
     uint64_t grid = (uint64_t)h->nsm * per_sm;
-    grid = std::min<uint64_t>(grid, (n + block - 1) / block);
+    grid = lat ? std::min<uint64_t>(grid, items) : std::min<uint64_t>(grid, (n + block - 1) / block);
     NMC_CUDA(h, nmc::launch_mcsub(p, trace, (int)grid, block, h->stream));
   } else {
     nmc::XyzParams p = h->xp;

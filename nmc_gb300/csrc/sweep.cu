@@ -160,9 +160,9 @@ __global__ void __launch_bounds__(256, 3) sweep_kernel(const SweepParams P) {
       costheta = 2.f * dr.a - 1.f;
     else
       costheta = hg_sample<FAST>(ph, dr.a);
-    SpinTrig trig;
+    const SpinTrig trig = spin_trig<FAST>(costheta, TT ? dr.c : dr.b);
     float nx, ny, nz;
-    const bool vertical = spin_try<FAST>(costheta, TT ? dr.c : dr.b, ux, uy, uz, trig, nx, ny, nz);
+    const bool vertical = spin_try(costheta, trig, ux, uy, uz, nx, ny, nz);
     ++nsc;
     if (__builtin_expect(vertical | need_roul, 0)) {
       if (vertical) spin_vertical(costheta, trig, ux, uy, uz, nx, ny, nz);
