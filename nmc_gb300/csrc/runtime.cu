@@ -423,13 +423,14 @@ nmc_status launch(nmc_handle* h, uint64_t first, uint64_t n, nmc_photon_record* 
     p.n = n;
     p.trace = tr;
     block = h->ext.block_size > 0 ? h->ext.block_size : 512;
-    // Up to four photons per lane of the latency variant it is the faster one
-    // (semi-infinite medium, mua 1, mus 100: 1e4 photons 0.58 against 0.90 ms,
-    // 1e5 1.01 / 1.58, 3e5 1.71 / 1.82, 1e6 4.44 / 3.82 ms); below one photon
-    // per lane they are spread over all its warps.
+    // The latency variant where it pays (mua 1, mus 100: 1e4 photons take 0.58
+    // against 0.90 ms, 1e5 1.01 / 1.58, 3e5 1.71 / 1.82, 1e6 4.44 / 3.82 ms);
+    // below one photon per lane they are spread over all its warps.
     const uint64_t warps = (uint64_t)h->nsm * nmc::kLatBlocks * (nmc::kLatBlock / 32);
     const uint64_t items = (n + p.per_fetch - 1) / p.per_fetch;
-    const bool lat = !trace && h->ext.block_size <= 0 && h->ext.blocks_per_sm <= 0 && items <= warps * 128;
+    nmc::LatencyRule rule;
+    rule.add((double)n, p.mua, p.mus);
+    const bool lat = !trace && h->ext.block_size <= 0 && h->ext.blocks_per_sm <= 0 && rule.pays();
     if (lat) {
       block = nmc::kLatBlock;
       p.lanes = (unsigned int)std::min<uint64_t>(32, (items + warps - 1) / warps);
@@ -1211,13 +1212,22 @@ nmc_status nmc_run_sweep(nmc_handle* h, const nmc_sweep_set* sets, int32_t n_set
       // sums, e2, counter and J are contiguous: clear them together
       cudaMemsetAsync(p.sums, 0, al(b_sums) + al(b_e2) + al(b_work) + al(b_J), h->stream) != cudaSuccess)
     return fail(h, NMC_EDEVICE, "sweep buffer set-up");
+  const uint64_t warps = (uint64_t)h->nsm * nmc::kLatBlocks * (nmc::kLatBlock / 32);
+  // The latency variant where it pays: 351 long-lived sets of 200, 1e4 and 2e4
+  // photons take 12.4, 28.6 and 45.4 ms, against 20.3, 37.6 and 44.8 ms;
+  // short-lived ones of 1e3 photons take 1.4 against 1.5 ms, of 4e3 3.5 / 2.7.
+  nmc::LatencyRule rule;
+  for (int k = 0; k < n_sets; ++k) rule.add((double)sets[k].photons, sets[k].mua, sets[k].mus);
+  const bool lat = h->ext.block_size <= 0 && h->ext.blocks_per_sm <= 0 && rule.pays();
+  if (lat) p.lanes = (unsigned int)std::max<uint64_t>(1, std::min<uint64_t>(32, (p.total + warps - 1) / warps));
   const int block = h->ext.block_size > 0 ? h->ext.block_size : 256;
   int per_sm = 0;
   if (nmc::sweep_occupancy(p, block, &per_sm) != cudaSuccess || per_sm < 1)
     return fail(h, NMC_EDEVICE, "sweep kernel does not fit on an SM");
   if (h->ext.blocks_per_sm > 0) per_sm = std::min(per_sm, (int)h->ext.blocks_per_sm);
+  if (lat) per_sm = std::min(per_sm, nmc::kLatBlocks);
   uint64_t grid = (uint64_t)h->nsm * per_sm;
-  grid = std::max<uint64_t>(1, std::min<uint64_t>(grid, (p.total + block - 1) / block));
+  grid = std::max<uint64_t>(1, std::min<uint64_t>(grid, lat ? p.total : (p.total + block - 1) / block));
   EventPair ev = get_pair(h);
   cudaEventRecord(ev.a, h->stream);
   if (p.total > 0 && nmc::launch_sweep(p, (int)grid, block, h->stream) != cudaSuccess)

@@ -23,7 +23,8 @@
 // of 1.4e7 photons in 71.0 ms, against 92.3 ms with the table reads at 4
 // blocks (and 85.6 ms with the constants in registers squeezed to 4 blocks);
 // 3.5e6 photons, where fewer resident photons also shorten the tail, 37.6
-// against 53.8 ms.
+// against 53.8 ms.  Sweeps whose tail outweighs their work take the latency
+// variant (99 registers, thin warps): the 3.5e6 photons 28.6 ms.
 #include <cuda_runtime.h>
 
 #include "engine.h"
@@ -31,13 +32,16 @@
 namespace nmc {
 namespace {
 
-template <int PHASE, bool FAST>
-__global__ void __launch_bounds__(256, 3) sweep_kernel(const SweepParams P) {
+// LAT: the latency variant (engine.h).
+template <int PHASE, bool FAST, bool LAT>
+__global__ void __launch_bounds__(kLatBlock, LAT ? kLatBlocks : 3) sweep_kernel(const SweepParams P) {
   using M = Math<FAST>;
   constexpr bool TT = PHASE == kPhaseTT;
   extern __shared__ unsigned long long s_sum[];  // nsets x 5: photons, hops, S, A, E
   double* s_e2 = reinterpret_cast<double*>(s_sum + 5 * P.nsets);
+  __shared__ int s_idle[LAT ? kLatBlock / 32 : 1];  // lanes of each warp that found the queue empty
   for (int k = threadIdx.x; k < 6 * P.nsets; k += blockDim.x) s_sum[k] = 0ull;
+  if (LAT && threadIdx.x < kLatBlock / 32) s_idle[threadIdx.x] = 0;
   __syncthreads();
   const int BINS = P.bins;
   const uint32_t k0 = P.k0;
@@ -49,23 +53,67 @@ __global__ void __launch_bounds__(256, 3) sweep_kernel(const SweepParams P) {
   float mut = 1.f, oma = 0.f;
   PhaseConst ph;
   uint32_t nsc = 0, nsub = 0, k1 = P.k1;
-  int set = 0;
-  const SweepSetDev* S = P.sets;
+  int set = 0, slot = 0;
   bool alive = false, have = false;
 
-  while (true) {
-    if (!alive) {
-      if (have) {
-        unsigned long long* b = s_sum + 5 * set;
-        atomicAdd(b + 0, 1ull);
-        atomicAdd(b + 1, (unsigned long long)nsub);
-        atomicAdd(b + 2, to_fix(rsp));
-        atomicAdd(b + 3, to_fix(Atot));
-        atomicAdd(b + 4, to_fix(E));
-        if (E > 0.f) atomicAdd(s_e2 + set, (double)E * (double)E);
+  auto retire = [&]() {
+    unsigned long long* b = s_sum + 5 * set;
+    atomicAdd(b + 0, 1ull);
+    atomicAdd(b + 1, (unsigned long long)nsub);
+    atomicAdd(b + 2, to_fix(rsp));
+    atomicAdd(b + 3, to_fix(Atot));
+    atomicAdd(b + 4, to_fix(E));
+    if (E > 0.f) atomicAdd(s_e2 + set, (double)E * (double)E);
+  };
+  // HOP (:183-187) by s and ESCAPE (:190-214): true when the photon left
+  auto hop = [&](float s) {
+    x = fmaf(s, ux, x);
+    y = fmaf(s, uy, y);
+    z = fmaf(s, uz, z);
+    ++nsub;
+    if (P.boundaryflag == 1 && z <= P.zs) {
+      float uz1;
+      const SweepSetDev* S = P.sets + slot;
+      if (rng.fres_u(k0, k1) > rfresnel(__ldg(&S->n1), __ldg(&S->n2), -uz, &uz1)) {
+        x = fmaf(-s, ux, x);
+        y = fmaf(-s, uy, y);
+        z = fmaf(-s, uz, z);
+        const float s2 = fabsf(z / uz);
+        x = fmaf(s2, ux, x);
+        y = fmaf(s2, uy, y);
+        const float r = sqrtf(x * x + y * y);
+        int ir = (int)fminf(r * P.idr, (float)BINS) + 1;
+        if (ir > BINS) ir = BINS;
+        if (P.J) atomicAdd(P.J + (size_t)set * (BINS + 1) + ir, to_fix(W));
+        E += W;
+        return true;
       }
+      z = -z;
+      uz = -uz;
+    }
+    return false;
+  };
+  auto drop = [&]() {  // DROP (:224-234): absorbed weight only (no F(r,z) in sweeps)
+    const float absorb = W * oma;
+    W -= absorb;
+    Atot += absorb;
+  };
+  auto phase = [](const PhaseConst& q, float a, float b) {  // cos(theta)
+    if (PHASE == kPhaseTT) return tt_sample_param<FAST>(q, a, b);
+    if (PHASE == kPhaseIsoRef) return 2.f * a - 1.f;
+    return hg_sample<FAST>(q, a);
+  };
+
+  const bool idle = LAT && (threadIdx.x & 31) >= P.lanes;
+  while (!idle) {
+    if (!alive) {
+      if (have) retire();
+      have = false;
       const unsigned long long g = next_photon(P.work);
-      if (g >= P.total) break;
+      if (g >= P.total) {
+        if (LAT) atomicAdd(&s_idle[threadIdx.x >> 5], 1);
+        break;
+      }
       have = true;
       // queue slot of global photon g: prefix[k] <= g < prefix[k + 1]
       int lo = 0, hi = P.nsets;
@@ -73,7 +121,8 @@ __global__ void __launch_bounds__(256, 3) sweep_kernel(const SweepParams P) {
         const int mid = (lo + hi) >> 1;
         if (__ldg(P.prefix + mid) <= g) lo = mid; else hi = mid;
       }
-      S = P.sets + lo;
+      slot = lo;
+      const SweepSetDev* S = P.sets + lo;
       set = (int)__ldg(&S->id);
       k1 = P.k1 + (uint32_t)set;
       rng.init(__ldg(&S->first) + (g - __ldg(P.prefix + lo)));
@@ -120,57 +169,31 @@ __global__ void __launch_bounds__(256, 3) sweep_kernel(const SweepParams P) {
       alive = true;
     }
 
-    // ---- HOP (:183-187)
-    const float s = M::div(M::neglog(step_u), mut);
-    x = fmaf(s, ux, x);
-    y = fmaf(s, uy, y);
-    z = fmaf(s, uz, z);
-    ++nsub;
-    if (P.boundaryflag == 1 && z <= P.zs) {  // ESCAPE (:190-214)
-      float uz1;
-      if (rng.fres_u(k0, k1) > rfresnel(__ldg(&S->n1), __ldg(&S->n2), -uz, &uz1)) {
-        x = fmaf(-s, ux, x);
-        y = fmaf(-s, uy, y);
-        z = fmaf(-s, uz, z);
-        const float s2 = fabsf(z / uz);
-        x = fmaf(s2, ux, x);
-        y = fmaf(s2, uy, y);
-        const float r = sqrtf(x * x + y * y);
-        int ir = (int)fminf(r * P.idr, (float)BINS) + 1;
-        if (ir > BINS) ir = BINS;
-        if (P.J) atomicAdd(P.J + (size_t)set * (BINS + 1) + ir, to_fix(W));
-        E += W;
-        alive = false;
-        continue;
-      }
-      z = -z;
-      uz = -uz;
+    if (hop(M::div(M::neglog(step_u), mut))) {
+      alive = false;
+      continue;
     }
-    // ---- DROP (:224-234): absorbed weight only (no F(r,z) in sweeps)
-    const float absorb = W * oma;
-    W -= absorb;
-    Atot += absorb;
+    drop();
     // ---- SPIN (:243-279), ROULETTE (:289-294), next HOP's draw
     const bool need_roul = W < kTHRESHOLD;
     const SpinDraws dr = rng.spin_draws(need_roul, k0, k1);
-    float costheta;
-    if (PHASE == kPhaseTT)
-      costheta = tt_sample_param<FAST>(ph, dr.a, dr.b);
-    else if (PHASE == kPhaseIsoRef)
-      costheta = 2.f * dr.a - 1.f;
-    else
-      costheta = hg_sample<FAST>(ph, dr.a);
+    const float costheta = phase(ph, dr.a, dr.b);
     const SpinTrig trig = spin_trig<FAST>(costheta, TT ? dr.c : dr.b);
     float nx, ny, nz;
     const bool vertical = spin_try(costheta, trig, ux, uy, uz, nx, ny, nz);
     ++nsc;
-    if (__builtin_expect(vertical | need_roul, 0)) {
+    bool leave = false;
+    if (__builtin_expect(vertical | need_roul | (LAT && nsc % kThinLook == 0), 0)) {
       if (vertical) spin_vertical(costheta, trig, ux, uy, uz, nx, ny, nz);
       if (need_roul) {
         if (dr.roul <= kCHANCE)
           W /= kCHANCE;
         else
           alive = false;
+      }
+      if (LAT) {  // go on thin: the queue is empty and few lanes have a photon
+        const int none = *(volatile int*)&s_idle[threadIdx.x >> 5];
+        leave = (int)P.lanes - none <= kThinPhotons && (none > 0 || *(volatile unsigned long long*)P.work >= P.total);
       }
     }
     ux = nx;
@@ -181,6 +204,69 @@ __global__ void __launch_bounds__(256, 3) sweep_kernel(const SweepParams P) {
       alive = false;
       atomicOr(P.flags, (unsigned int)NMC_DEVFLAG_STEPCAP);
     }
+    if (LAT && leave && alive) break;
+  }
+
+  if constexpr (LAT) {
+    // the lanes without a photon compute the random part of the coming hops
+    const unsigned int lane = threadIdx.x & 31, all = 0xFFFFFFFFu;
+    float s = alive ? M::div(M::neglog(step_u), mut) : 0.f;
+    unsigned int mask;
+    while ((mask = __ballot_sync(all, alive)) != 0) {
+      const int n = __popc(mask), per = 32 / n;  // photons, and hops of each in this pass
+      const int first = __popc(mask & ((1u << lane) - 1u)) * per;  // my photon's first record
+      const int q = (int)lane / per, src = (int)__fns(mask, 0, min(q, n - 1) + 1);
+      const uint32_t plo = __shfl_sync(all, rng.plo, src), phi = __shfl_sync(all, rng.phi, src);
+      const uint32_t h = __shfl_sync(all, nsc, src) + 1u + (lane - q * per), key = __shfl_sync(all, k1, src);
+      const SweepSetDev* S = P.sets + __shfl_sync(all, slot, src);
+      const uint4 b = philox4x32_10(make_uint4(plo, phi, h, kPhiloxTag), k0, key);
+      const float r_cos = phase(S->ph, u01(b.x), u01(b.y));
+      const SpinTrig r_trig = spin_trig<FAST>(r_cos, TT ? u01(b.z) : u01(b.y));
+      const float r_s = M::div(M::neglog(u01(b.w)), __ldg(&S->mut));
+      for (int o = 0; o < per; ++o) {
+        const int k = first + o;
+        const float costheta = __shfl_sync(all, r_cos, k);
+        SpinTrig trig;
+        trig.sintheta = __shfl_sync(all, r_trig.sintheta, k);
+        trig.sinpsi = __shfl_sync(all, r_trig.sinpsi, k);
+        trig.cospsi = __shfl_sync(all, r_trig.cospsi, k);
+        const float s_next = __shfl_sync(all, r_s, k);
+        const float roul = TT ? 0.f : u01(__shfl_sync(all, b.z, k));
+        if (!alive) continue;
+        rng.hop = nsc;
+        if (hop(s)) {
+          alive = false;
+          continue;
+        }
+        drop();
+        float nx, ny, nz;
+        const bool vertical = spin_try(costheta, trig, ux, uy, uz, nx, ny, nz);
+        ++nsc;
+        const bool need_roul = W < kTHRESHOLD;
+        if (__builtin_expect(vertical | need_roul, 0)) {
+          if (vertical) spin_vertical(costheta, trig, ux, uy, uz, nx, ny, nz);
+          if (need_roul) {
+            const float u = TT ? u01(rng.block(nsc | 0x40000000u, k0, k1).x) : roul;
+            if (u <= kCHANCE)
+              W /= kCHANCE;
+            else
+              alive = false;
+          }
+        }
+        ux = nx;
+        uy = ny;
+        uz = nz;
+        s = s_next;
+        if (alive && nsub >= P.step_cap) {
+          alive = false;
+          atomicOr(P.flags, (unsigned int)NMC_DEVFLAG_STEPCAP);
+        }
+      }
+      if (have && !alive) {
+        retire();
+        have = false;
+      }
+    }
   }
 
   __syncthreads();
@@ -190,11 +276,11 @@ __global__ void __launch_bounds__(256, 3) sweep_kernel(const SweepParams P) {
     if (s_e2[k] != 0.0) atomicAdd(P.e2 + k, s_e2[k]);
 }
 
-template <bool FAST>
+template <bool FAST, bool LAT>
 const void* pick(int phase) {
-  if (phase == kPhaseTT) return (const void*)sweep_kernel<kPhaseTT, FAST>;
-  if (phase == kPhaseIsoRef) return (const void*)sweep_kernel<kPhaseIsoRef, FAST>;
-  return (const void*)sweep_kernel<kPhaseHG, FAST>;
+  if (phase == kPhaseTT) return (const void*)sweep_kernel<kPhaseTT, FAST, LAT>;
+  if (phase == kPhaseIsoRef) return (const void*)sweep_kernel<kPhaseIsoRef, FAST, LAT>;
+  return (const void*)sweep_kernel<kPhaseHG, FAST, LAT>;
 }
 
 }  // namespace
@@ -202,7 +288,10 @@ const void* pick(int phase) {
 size_t sweep_smem_bytes(int nsets) { return (size_t)nsets * 6 * 8; }
 
 cudaError_t sweep_prepare(const SweepParams& p, const void** f, size_t* sh) {
-  *f = p.fast ? pick<true>(p.phase_kind) : pick<false>(p.phase_kind);
+  if (p.lanes > 0)
+    *f = p.fast ? pick<true, true>(p.phase_kind) : pick<false, true>(p.phase_kind);
+  else
+    *f = p.fast ? pick<true, false>(p.phase_kind) : pick<false, false>(p.phase_kind);
   *sh = sweep_smem_bytes(p.nsets);
   if (*sh > 48 * 1024) return cudaFuncSetAttribute(*f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)*sh);
   return cudaSuccess;
