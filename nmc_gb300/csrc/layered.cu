@@ -96,6 +96,7 @@ struct LayParams {
   unsigned long long* work;
   unsigned int* flags;
   uint32_t step_cap;
+  unsigned int lanes;  // latency variant: lanes of a warp that take photons
   // adjoint
   const float* g_rd;  // nr + 1 upstream gradient of rd_r (may be null)
   const float* g_tt;  // nr + 1 upstream gradient of tt_r (may be null)
@@ -105,12 +106,15 @@ struct LayParams {
   int iso;            // isotropic scattering (the reference's mcsub sampling)
 };
 
-template <bool FAST, bool ADJ, bool REF>
-__global__ void __launch_bounds__(256, 4) layered_kernel(const LayParams P) {
+// LAT: the latency variant (engine.h)
+template <bool FAST, bool ADJ, bool REF, bool LAT>
+__global__ void __launch_bounds__(kLatBlock, LAT ? kLatBlocks : 4) layered_kernel(const LayParams P) {
   using M = Math<FAST>;
   __shared__ LayDev s_lay[kMaxLayers];
   __shared__ double s_sum[NMC_LAY_FIELDS];
   __shared__ double s_grad[ADJ ? 3 * kMaxAdjLayers : 1];
+  __shared__ int s_idle[LAT ? kLatBlock / 32 : 1];  // lanes of each warp that found the queue empty
+  if (LAT && threadIdx.x < kLatBlock / 32) s_idle[threadIdx.x] = 0;
   // absorbed weight per layer, then (if it fits) A(z): block-private u64
   // fixed-point sums, added to the global tallies once at the end; every
   // interaction deposits, and a handful of global addresses would serialise
@@ -143,107 +147,78 @@ __global__ void __launch_bounds__(256, 4) layered_kernel(const LayParams P) {
     return uz > 0.f ? (s_lay[L].z1 - z) / uz : (uz < 0.f ? (s_lay[L].z0 - z) / uz : INFINITY);
   };
 
-  while (true) {
-    if (!alive) {
-      if (have) {
-        if (dep_w > 0.f && idx_ok(dep_l, (unsigned)P.nl, P.flags)) atomicAdd(s_al + dep_l, to_fix(dep_w));
-        atomicAdd(&s_sum[NMC_LAY_PHOTONS], 1.0);
-        atomicAdd(&s_sum[NMC_LAY_RD], (double)rd);
-        atomicAdd(&s_sum[NMC_LAY_RD2], (double)rd * (double)rd);
-        atomicAdd(&s_sum[NMC_LAY_TT], (double)tt);
-        atomicAdd(&s_sum[NMC_LAY_TT2], (double)tt * (double)tt);
-        atomicAdd(&s_sum[NMC_LAY_INTERACTIONS], (double)hop);
-        if (ADJ && score != 0.f)
-          for (int l = 0; l < P.nl; ++l) {
-            atomicAdd(&s_grad[l], (double)(-score * aL[l]));
-            atomicAdd(&s_grad[kMaxAdjLayers + l],
-                      (double)(score * (s_lay[l].mus > 0.f ? aN[l] / s_lay[l].mus - aL[l] : -aL[l])));
-            atomicAdd(&s_grad[2 * kMaxAdjLayers + l], (double)(score * aQ[l]));
-          }
+  auto retire = [&]() {
+    if (dep_w > 0.f && idx_ok(dep_l, (unsigned)P.nl, P.flags)) atomicAdd(s_al + dep_l, to_fix(dep_w));
+    atomicAdd(&s_sum[NMC_LAY_PHOTONS], 1.0);
+    atomicAdd(&s_sum[NMC_LAY_RD], (double)rd);
+    atomicAdd(&s_sum[NMC_LAY_RD2], (double)rd * (double)rd);
+    atomicAdd(&s_sum[NMC_LAY_TT], (double)tt);
+    atomicAdd(&s_sum[NMC_LAY_TT2], (double)tt * (double)tt);
+    atomicAdd(&s_sum[NMC_LAY_INTERACTIONS], (double)hop);
+    if (ADJ && score != 0.f)
+      for (int l = 0; l < P.nl; ++l) {
+        atomicAdd(&s_grad[l], (double)(-score * aL[l]));
+        atomicAdd(&s_grad[kMaxAdjLayers + l],
+                  (double)(score * (s_lay[l].mus > 0.f ? aN[l] / s_lay[l].mus - aL[l] : -aL[l])));
+        atomicAdd(&s_grad[2 * kMaxAdjLayers + l], (double)(score * aQ[l]));
       }
-      const unsigned long long g = next_photon(P.work);
-      if (g >= P.n) break;
-      have = true;
-      alive = true;
-      const unsigned long long pid = P.first + g;
-      c0 = (uint32_t)pid, c1 = (uint32_t)(pid >> 32);
-      x = y = z = ux = uy = 0.f;
-      uz = 1.f;
-      w = P.w0;
-      L = dep_l = 0;
-      hop = ev = 0;
-      rd = tt = dep_w = score = 0.f;
-      if (ADJ)
-        for (int l = 0; l < P.nl; ++l) aL[l] = aN[l] = aQ[l] = 0.f;
-      if (REF) {
-        tr.init_photon(pid, P.batch, false, false);
-        tr.next();  // the launch draw (radius 0: the beam stays on the axis)
-      } else {
-        r = philox4x32_10(make_uint4(c0, c1, 0u, kLayTag), RoundKeys{P.rk});
-      }
-      sleft = M::neglog(REF ? tr.step_draw() : u01(r.x));
-    }
-
-    float s = path();
-    // A step reaches the boundary when s >= distance / uz.  Most do not come
-    // near it, which a product shows: only the others divide.  (The product
-    // and the quotient are within 2^-22 of the exact values.)
+  };
+  // A step reaches the boundary when s >= distance / uz.  Most do not come
+  // near it, which a product shows: only the others divide.  (The product and
+  // the quotient are within 2^-22 of the exact values.)
+  auto near = [&](float s) {
     const float dz = uz > 0.f ? s_lay[L].z1 - z : z - s_lay[L].z0;
-    if (!(s * fabsf(uz) * 1.000001f < dz)) {
-      const float db = ahead();
-      if (s >= db) {  // reaches the boundary: CROSS
-        const LayDev& Ly = s_lay[L];
-        x = fmaf(db, ux, x);
-        y = fmaf(db, uy, y);
-        z = uz > 0.f ? Ly.z1 : Ly.z0;
-        if (ADJ) aL[L] += db;
-        sleft = Ly.inv_mut > 0.f ? fmaxf(sleft - db / Ly.inv_mut, 0.f) : sleft;
-        const bool down = uz > 0.f;
-        const int Ln = down ? L + 1 : L - 1;
-        const float nt = Ln < 0 ? P.n_above : (Ln >= P.nl ? P.n_below : s_lay[Ln].n);
-        float uzt = 0.f;
-        const float R = rfresnel(Ly.n, nt, fabsf(uz), &uzt);
-        // a draw lies in (0, 1): matched layers and total reflection need none
-        bool reflect = R >= 1.f;
-        if (REF)
-          reflect = tr.next() <= R;
-        else if (R > 0.f && R < 1.f)
-          reflect = u01(philox4x32_10(make_uint4(c0, c1, ev | 0x80000000u, kLayTag), RoundKeys{P.rk}).x) <= R;
-        ++ev;
-        if (reflect) {
-          uz = -uz;
-        } else if (Ln < 0 || Ln >= P.nl) {  // escapes
-          const float rr = sqrtf(x * x + y * y);
-          const int ir = min((int)(rr * P.idr), P.nr);
-          if (Ln < 0) {
-            if (idx_ok(ir, (unsigned)P.nr + 1u, P.flags)) atomicAdd(P.rd_r + ir, to_fix(w));
-            rd += w;
-            if (ADJ && P.g_rd) score = w * __ldg(P.g_rd + ir);
-          } else {
-            if (idx_ok(ir, (unsigned)P.nr + 1u, P.flags)) atomicAdd(P.tt_r + ir, to_fix(w));
-            tt += w;
-            if (ADJ && P.g_tt) score = w * __ldg(P.g_tt + ir);
-          }
-          alive = false;
-        } else {  // refracted into the next layer (Snell)
-          const float ratio = Ly.n / nt;
-          ux *= ratio;
-          uy *= ratio;
-          uz = down ? uzt : -uzt;
-          L = Ln;
-        }
-        if (ev > P.step_cap) {
-          atomicOr(P.flags, (unsigned int)NMC_DEVFLAG_STEPCAP);
-          alive = false;
-        }
-        if (alive) {  // go on from the boundary: most steps now end inside the layer
-          if (sleft <= 0.f) sleft = M::neglog(REF ? tr.step_draw() : u01(r.x));
-          s = path();
-        }
-        if (!alive || s >= ahead()) continue;
+    return !(s * fabsf(uz) * 1.000001f < dz);
+  };
+  auto cross = [&](float db) {  // CROSS, db ahead
+    const LayDev& Ly = s_lay[L];
+    x = fmaf(db, ux, x);
+    y = fmaf(db, uy, y);
+    z = uz > 0.f ? Ly.z1 : Ly.z0;
+    if (ADJ) aL[L] += db;
+    sleft = Ly.inv_mut > 0.f ? fmaxf(sleft - db / Ly.inv_mut, 0.f) : sleft;
+    const bool down = uz > 0.f;
+    const int Ln = down ? L + 1 : L - 1;
+    const float nt = Ln < 0 ? P.n_above : (Ln >= P.nl ? P.n_below : s_lay[Ln].n);
+    float uzt = 0.f;
+    const float R = rfresnel(Ly.n, nt, fabsf(uz), &uzt);
+    // a draw lies in (0, 1): matched layers and total reflection need none
+    bool reflect = R >= 1.f;
+    if (REF)
+      reflect = tr.next() <= R;
+    else if (R > 0.f && R < 1.f)
+      reflect = u01(philox4x32_10(make_uint4(c0, c1, ev | 0x80000000u, kLayTag), RoundKeys{P.rk}).x) <= R;
+    ++ev;
+    if (reflect) {
+      uz = -uz;
+    } else if (Ln < 0 || Ln >= P.nl) {  // escapes
+      const float rr = sqrtf(x * x + y * y);
+      const int ir = min((int)(rr * P.idr), P.nr);
+      if (Ln < 0) {
+        if (idx_ok(ir, (unsigned)P.nr + 1u, P.flags)) atomicAdd(P.rd_r + ir, to_fix(w));
+        rd += w;
+        if (ADJ && P.g_rd) score = w * __ldg(P.g_rd + ir);
+      } else {
+        if (idx_ok(ir, (unsigned)P.nr + 1u, P.flags)) atomicAdd(P.tt_r + ir, to_fix(w));
+        tt += w;
+        if (ADJ && P.g_tt) score = w * __ldg(P.g_tt + ir);
       }
+      alive = false;
+    } else {  // refracted into the next layer (Snell)
+      const float ratio = Ly.n / nt;
+      ux *= ratio;
+      uy *= ratio;
+      uz = down ? uzt : -uzt;
+      L = Ln;
     }
-    // interaction inside the layer: HOP, DROP, SPIN, ROULETTE
+    if (ev > P.step_cap) {
+      atomicOr(P.flags, (unsigned int)NMC_DEVFLAG_STEPCAP);
+      alive = false;
+    }
+  };
+  // the interaction after a path of s inside the layer: HOP, DROP, SPIN,
+  // ROULETTE; true where the photon is to look whether its warp goes on thin
+  auto interact = [&](float s, float ucos, float sinpsi, float cospsi, float uroul) {
     const LayDev& Ly = s_lay[L];
     x = fmaf(s, ux, x);
     y = fmaf(s, uy, y);
@@ -274,16 +249,15 @@ __global__ void __launch_bounds__(256, 4) layered_kernel(const LayParams P) {
           atomicAdd(P.a_rz + (size_t)ir * (P.nz + 1) + iz, fa);
       }
     }
-    const float ucos = REF ? tr.next() : u01(r.y);
     const float cth = P.iso ? 2.f * ucos - 1.f : hg_sample<FAST>(Ly.ph, ucos);
     if (ADJ && Ly.ph.hg_mode == 0) aQ[L] += dln_hg_dg(Ly.g, cth);
-    const SpinTrig trig = spin_trig<FAST>(cth, REF ? tr.next() : u01(r.z));
+    const SpinTrig trig{M::sqrt(fmaxf(fmaf(-cth, cth, 1.f), 0.f)), sinpsi, cospsi};
     float nx, ny, nz;
     const bool vertical = spin_try(cth, trig, ux, uy, uz, nx, ny, nz);
     ++hop;
     // the rare events of an interaction behind one test
-    const bool other = L != dep_l, carry = old + dep < old;
-    if (__builtin_expect(vertical | other | carry | (w < kTHRESHOLD) | (hop > P.step_cap), 0)) {
+    const bool other = L != dep_l, carry = old + dep < old, look = LAT && hop % kThinLook == 0;
+    if (__builtin_expect(vertical | other | carry | look | (w < kTHRESHOLD) | (hop > P.step_cap), 0)) {
       if (carry) atomicAdd(reinterpret_cast<unsigned int*>(s_az + iz) + 1, 1u);
       if (vertical) spin_vertical(cth, trig, ux, uy, uz, nx, ny, nz);
       if (other && absorb > 0.f) {
@@ -292,7 +266,7 @@ __global__ void __launch_bounds__(256, 4) layered_kernel(const LayParams P) {
         dep_w = 0.f;
       }
       if (w < kTHRESHOLD) {
-        if ((REF ? tr.next() : u01(r.w)) <= kCHANCE)
+        if ((REF ? tr.next() : uroul) <= kCHANCE)
           w /= kCHANCE;
         else
           alive = false;
@@ -306,8 +280,101 @@ __global__ void __launch_bounds__(256, 4) layered_kernel(const LayParams P) {
     ux = nx;
     uy = ny;
     uz = nz;
+    return look;
+  };
+
+  const bool idle = LAT && (threadIdx.x & 31) >= P.lanes;
+  while (!idle) {
+    if (!alive) {
+      if (have) retire();
+      have = false;
+      const unsigned long long g = next_photon(P.work);
+      if (g >= P.n) {
+        if (LAT) atomicAdd(&s_idle[threadIdx.x >> 5], 1);
+        break;
+      }
+      have = true;
+      alive = true;
+      const unsigned long long pid = P.first + g;
+      c0 = (uint32_t)pid, c1 = (uint32_t)(pid >> 32);
+      x = y = z = ux = uy = 0.f;
+      uz = 1.f;
+      w = P.w0;
+      L = dep_l = 0;
+      hop = ev = 0;
+      rd = tt = dep_w = score = 0.f;
+      if (ADJ)
+        for (int l = 0; l < P.nl; ++l) aL[l] = aN[l] = aQ[l] = 0.f;
+      if (REF) {
+        tr.init_photon(pid, P.batch, false, false);
+        tr.next();  // the launch draw (radius 0: the beam stays on the axis)
+      } else {
+        r = philox4x32_10(make_uint4(c0, c1, 0u, kLayTag), RoundKeys{P.rk});
+      }
+      sleft = M::neglog(REF ? tr.step_draw() : u01(r.x));
+    }
+
+    float s = path();
+    if (near(s)) {
+      const float db = ahead();
+      if (s >= db) {
+        cross(db);
+        if (alive) {  // go on from the boundary: most steps now end inside the layer
+          if (sleft <= 0.f) sleft = M::neglog(REF ? tr.step_draw() : u01(r.x));
+          s = path();
+        }
+        if (!alive || s >= ahead()) continue;
+      }
+    }
+    const float ucos = REF ? tr.next() : u01(r.y);
+    float sinpsi, cospsi;
+    M::sincos2pi(REF ? tr.next() : u01(r.z), &sinpsi, &cospsi);
+    const bool look = interact(s, ucos, sinpsi, cospsi, u01(r.w));
     if (!REF) r = philox4x32_10(make_uint4(c0, c1, hop, kLayTag), RoundKeys{P.rk});
     if (!REF || alive) sleft = M::neglog(REF ? tr.step_draw() : u01(r.x));
+    if (LAT && look && alive) {  // go on thin: the queue is empty and few lanes have a photon
+      const int none = *(volatile int*)&s_idle[threadIdx.x >> 5];
+      if ((int)P.lanes - none <= kThinPhotons && (none > 0 || *(volatile unsigned long long*)P.work >= P.n)) break;
+    }
+  }
+
+  if constexpr (LAT) {
+    // the lanes without a photon compute the random part of the coming interactions
+    const unsigned int lane = threadIdx.x & 31, all = 0xFFFFFFFFu;
+    unsigned int mask;
+    while ((mask = __ballot_sync(all, alive)) != 0) {
+      const int n = __popc(mask), per = 32 / n;  // photons, and interactions of each in this pass
+      const int first = __popc(mask & ((1u << lane) - 1u)) * per;  // my photon's first record
+      const int q = (int)lane / per, src = (int)__fns(mask, 0, min(q, n - 1) + 1);
+      const uint32_t p0 = __shfl_sync(all, c0, src), p1 = __shfl_sync(all, c1, src);
+      const uint32_t h = __shfl_sync(all, hop, src) + (lane - q * per);
+      const uint4 b = philox4x32_10(make_uint4(p0, p1, h, kLayTag), RoundKeys{P.rk});
+      const float r_step = M::neglog(u01(b.x));
+      float r_sin, r_cos;
+      M::sincos2pi(u01(b.z), &r_sin, &r_cos);
+      for (int o = 0; o < per; ++o) {
+        const int k = first + o;
+        const float step = __shfl_sync(all, r_step, k), ucos = u01(__shfl_sync(all, b.y, k));
+        const float sinpsi = __shfl_sync(all, r_sin, k), cospsi = __shfl_sync(all, r_cos, k);
+        const float uroul = u01(__shfl_sync(all, b.w, k));
+        if (!alive) continue;
+        sleft = step;
+        float s = path();
+        while (near(s)) {
+          const float db = ahead();
+          if (!(s >= db)) break;
+          cross(db);
+          if (!alive) break;
+          if (sleft <= 0.f) sleft = step;
+          s = path();
+        }
+        if (alive) interact(s, ucos, sinpsi, cospsi, uroul);
+      }
+      if (have && !alive) {
+        retire();
+        have = false;
+      }
+    }
   }
   __syncthreads();
   for (int i = threadIdx.x; i < n_priv; i += blockDim.x) {
@@ -444,23 +511,32 @@ nmc_status layered_impl(int32_t device, const nmc_layered_config* cfg, const nmc
   P.batch = ref ? c.seed : 1;
   P.iso = iso ? 1 : 0;
   const bool fast = !(c.flags & NMC_FLAG_PRECISE_MATH);
-  const void* f =
-      adj ? (fast ? (const void*)layered_kernel<true, true, false> : (const void*)layered_kernel<false, true, false>)
-      : ref ? (fast ? (const void*)layered_kernel<true, false, true> : (const void*)layered_kernel<false, false, true>)
-            : (fast ? (const void*)layered_kernel<true, false, false> : (const void*)layered_kernel<false, false, false>);
+  int nsm = 0;
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device);
+  const unsigned long long warps = (unsigned long long)nsm * kLatBlocks * (kLatBlock / 32);
+  // Up to four photons per lane of the latency variant it is the faster one
+  // (three-layer skin: 1e3 photons 6.0 against 6.7 ms, 1e5 9.6 / 10.1, 3e5 14.1
+  // / 15.5, 1e6 24.7 / 20.8 ms); the reference's generator is sequential.
+  const bool lat = !ref && photons <= warps * 128;
+  P.lanes = (unsigned int)std::max<unsigned long long>(1, std::min<unsigned long long>(32, (photons + warps - 1) / warps));
+#define NMC_LAYERED(ADJ, REF, LAT) \
+  (fast ? (const void*)layered_kernel<true, ADJ, REF, LAT> : (const void*)layered_kernel<false, ADJ, REF, LAT>)
+  const void* f = adj   ? (lat ? NMC_LAYERED(true, false, true) : NMC_LAYERED(true, false, false))
+                  : ref ? NMC_LAYERED(false, true, false)
+                        : (lat ? NMC_LAYERED(false, false, true) : NMC_LAYERED(false, false, false));
+#undef NMC_LAYERED
   // A(z) joins the per-layer sums in shared memory while both fit in 16 KB
   // and every deposit is below 1 (no pure absorber under a whole weight)
   float most = 0.f;
   for (const LayDev& d : lay) most = std::max(most, P.w0 * d.mua * d.inv_mut);
   P.smem_az = (size_t)(c.n_layers + nz1) * 8 <= 16384 && most < 1.f ? 1 : 0;
   const size_t smem = (size_t)(c.n_layers + (P.smem_az ? nz1 : 0)) * 8;
-  int per_sm = 0, nsm = 0;
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device);
+  int per_sm = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f, 256, smem) != cudaSuccess || per_sm < 1)
     return done(NMC_EDEVICE);
-  const unsigned long long grid =
-      std::max<unsigned long long>(1, std::min<unsigned long long>((unsigned long long)nsm * per_sm,
-                                                                   (photons + 255) / 256));
+  if (lat) per_sm = std::min(per_sm, kLatBlocks);
+  const unsigned long long grid = std::max<unsigned long long>(
+      1, std::min<unsigned long long>((unsigned long long)nsm * per_sm, lat ? photons : (photons + 255) / 256));
   void* args[] = {(void*)&P};
   if (photons > 0 && cudaLaunchKernel(f, dim3((unsigned)grid), dim3(256), args, smem, st) != cudaSuccess)
     return done(NMC_EDEVICE);
