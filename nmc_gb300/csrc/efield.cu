@@ -107,17 +107,28 @@ struct EfParams {
   unsigned long long* work;
   unsigned int* flags;
   uint32_t step_cap;
+  unsigned int lanes;  // latency variant: lanes of a warp that take photons
   nmc_speckle* spk;  // nsets * spk_max * map_n^2 records, or null
   int* spk_count;    // nsets * map_n^2 arrivals
   uint32_t spk_max;
 };
 
-__device__ __forceinline__ float2 cmul(float2 a, float2 b) {
-  return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
-}
 __device__ __forceinline__ float2 cmulc(float2 a, float2 b) {  // a conj(b)
   return make_float2(a.x * b.x + a.y * b.y, a.y * b.x - a.x * b.y);
 }
+// a b + c d and a b - c d with the first product fused.  A photon's path
+// depends on every rounding of its scatterings, so their sums of products are
+// written out: every form of the kernel then follows the same photons, whatever
+// the compiler would have fused there.
+__device__ __forceinline__ float dot2(float a, float b, float c, float d) { return __fmaf_rn(a, b, __fmul_rn(c, d)); }
+__device__ __forceinline__ float det2(float a, float b, float c, float d) { return __fmaf_rn(a, b, -__fmul_rn(c, d)); }
+__device__ __forceinline__ float dot3(float ax, float ay, float az, float bx, float by, float bz) {
+  return __fmaf_rn(az, bz, dot2(ax, bx, ay, by));
+}
+__device__ __forceinline__ float2 cmul_fused(float2 a, float2 b) {
+  return make_float2(det2(a.x, b.x, a.y, b.y), dot2(a.x, b.y, a.y, b.x));
+}
+__device__ __forceinline__ float norm2(float2 a) { return dot2(a.x, a.x, a.y, a.y); }
 __device__ __forceinline__ float cnorm(float2 a) { return a.x * a.x + a.y * a.y; }
 __device__ __forceinline__ float wrap_pi(float a) { return a - kTwoPi * rintf(a * (1.f / kTwoPi)); }
 
@@ -190,13 +201,16 @@ __device__ __forceinline__ void perp_of(float ux, float uy, float uz, float& px,
   }
 }
 
-template <bool FAST>
-__global__ void __launch_bounds__(256) efield_kernel(const EfParams P) {
+// LAT: the latency variant (engine.h)
+template <bool FAST, bool LAT>
+__global__ void __launch_bounds__(kLatBlock, LAT ? kLatBlocks : 4) efield_kernel(const EfParams P) {
   using M = Math<FAST>;
   extern __shared__ float s_cdf[];
   __shared__ double s_sum[kEfMaxSets * NMC_EF_FIELDS];
+  __shared__ int s_idle[LAT ? kLatBlock / 32 : 1];  // lanes of each warp that found the queue empty
   for (int i = threadIdx.x; i < 2 * P.n_angles; i += blockDim.x) s_cdf[i] = P.cdf[i];
   for (int i = threadIdx.x; i < P.nsets * NMC_EF_FIELDS; i += blockDim.x) s_sum[i] = 0.0;
+  if (LAT && threadIdx.x < kLatBlock / 32) s_idle[threadIdx.x] = 0;
   // guide to the inverse-CDF search: s_guide[m][k] = the bracket start of
   // u = k / kEfGuide, so a draw's bracket search spans a few entries instead
   // of all n_angles (the same bracket, found in fewer dependent steps)
@@ -215,170 +229,160 @@ __global__ void __launch_bounds__(256) efield_kernel(const EfParams P) {
   __syncthreads();
   const int MN = P.map_n * P.map_n, SN = P.sep_n * P.sep_n;
 
-  while (true) {
-    const unsigned long long g = next_photon(P.work);
-    if (g >= P.total) break;
-    int lo = 0, hi = P.nsets;
-    while (hi - lo > 1) {
-      const int mid = (lo + hi) >> 1;
-      if (__ldg(P.prefix + mid) <= g) lo = mid; else hi = mid;
-    }
-    const int set = lo;
-    const EfSet& S = P.sets[set];
-    const unsigned long long pid = S.first + (g - __ldg(P.prefix + set));
-    const uint32_t k1 = P.k1 + (uint32_t)set, c0 = (uint32_t)pid, c1 = (uint32_t)(pid >> 32);
-    double* sm = s_sum + set * NMC_EF_FIELDS;
-    atomicAdd(&sm[NMC_EF_PHOTONS], 1.0);
-    atomicAdd(&sm[NMC_EF_SPECULAR], (double)(1.f - S.w0));
+  float x = 0.f, y = 0.f, z = 0.f, ux = 0.f, uy = 0.f, uz = 1.f, px = 0.f, py = 1.f, pz = 0.f;
+  float2 T00 = make_float2(0.f, 0.f), T01 = T00, T10 = T00, T11 = T00;
+  float w = 0.f, fx = 0.f, fy = 0.f, lx = 0.f, ly = 0.f;
+  PathSum path;
+  int med = 0, set = 0;
+  unsigned int nsc = 0;
+  uint32_t hop = 0, k1 = 0, c0 = 0, c1 = 0;
+  bool alive = false, have = false, escaped = false;
+  double* sm = s_sum;
 
-    float x = 0.f, y = 0.f, z = 0.f, ux = S.ux, uy = S.uy, uz = S.uz, px = S.px, py = S.py, pz = S.pz;
-    float2 T00 = S.t[0], T01 = S.t[1], T10 = S.t[2], T11 = S.t[3];
-    float w = S.w0, fx = 0.f, fy = 0.f, lx = 0.f, ly = 0.f;
-    PathSum path;
-    int med = 0;
-    unsigned int nsc = 0;
-    uint32_t hop = 0;
-    bool alive = true, escaped = false;
-    while (alive) {
-      const uint4 r = philox4x32_10(make_uint4(c0, c1, hop, kEfTag), P.k0, k1);
-      const EfMedium& Md = P.med[med];
-      const float s = M::neglog(u01(r.x)) * Md.inv_mut;
-      if (uz < 0.f && z + s * uz < 0.f) {  // reaches the surface
-        const float d = -z / uz;
-        x = fmaf(d, ux, x);
-        y = fmaf(d, uy, y);
-        z = 0.f;
-        path.add(d);
-        float uzt;
-        const float rsp = rfresnel(P.n_medium, P.n_outside, -uz, &uzt);
-        const uint4 a = philox4x32_10(make_uint4(c0, c1, hop | 0x40000000u, kEfTag), P.k0, k1);
-        if (u01(a.x) > rsp) {
-          escaped = true;
-          break;
-        }
-        // mirrored; -M e_perp keeps the frame right-handed, so the perp row flips
-        uz = -uz;
-        px = -px;
-        py = -py;
-        T10 = make_float2(-T10.x, -T10.y);
-        T11 = make_float2(-T11.x, -T11.y);
-        const float rest = s - d;
-        x = fmaf(rest, ux, x);
-        y = fmaf(rest, uy, y);
-        z = rest * uz;
-        path.add(rest);
-      } else {
-        x = fmaf(s, ux, x);
-        y = fmaf(s, uy, y);
-        z = fmaf(s, uz, z);
-        path.add(s);
-      }
-      w *= Md.surv;
-      if (med == 0 && u01(r.w) < Md.p_raman) {  // Raman conversion
-        med = 1;
-        atomicAdd(&sm[NMC_EF_RAMAN_N], 1.0);
-        if (P.depth) {
-          const int b = (int)(z * P.depth_inv);
-          if (b >= 0 && b < P.depth_bins) atomicAdd(P.depth + (size_t)set * P.depth_bins + b, (double)w);
-        }
-        const float ct = 2.f * u01(r.y) - 1.f, st = sqrtf(fmaxf(0.f, 1.f - ct * ct));
-        float sp, cp;
-        M::sincos2pi(u01(r.z), &sp, &cp);
-        ux = st * cp;
-        uy = st * sp;
-        uz = ct;
-        perp_of(ux, uy, uz, px, py, pz);
-        T00 = make_float2(1.f, 0.f);
-        T01 = make_float2(0.f, 0.f);
-        T10 = make_float2(0.f, 0.f);
-        T11 = make_float2(1.f, 0.f);
-      } else {  // scattering
-        const float* cdf = s_cdf + Md.cdf_off;
-        const float uth = u01(r.y);
-        const unsigned int* gd = s_guide + med * (kEfGuide + 1);
-        const int gk = min((int)(uth * kEfGuide), kEfGuide - 1);
-        int a0 = (int)gd[gk], a1 = min((int)gd[gk + 1] + 1, P.n_angles - 1);
-        while (a1 - a0 > 1) {
-          const int mid = (a0 + a1) >> 1;
-          if (cdf[mid] <= uth) a0 = mid; else a1 = mid;
-        }
-        const float q0 = cdf[a0], q1 = cdf[a1];
-        const float fr = q1 > q0 ? fminf(fmaxf(M::div(uth - q0, q1 - q0), 0.f), 1.f) : 0.5f;
-        const float th = ((float)a0 + fr) * P.dtheta;
-        float sth, cth;
-        if (FAST) __sincosf(th, &sth, &cth); else sincosf(th, &sth, &cth);
-        const float4 A0 = __ldg(Md.S + a0), A1 = __ldg(Md.S + a1);
-        const float2 S1 = make_float2(fmaf(fr, A1.x - A0.x, A0.x), fmaf(fr, A1.y - A0.y, A0.y));
-        const float2 S2 = make_float2(fmaf(fr, A1.z - A0.z, A0.z), fmaf(fr, A1.w - A0.w, A0.w));
-        // azimuth from the field: p ∝ 1 + beta cos(2 phi - 2 phi0)
-        const float Pp = cnorm(T00) + cnorm(T01), Qp = cnorm(T10) + cnorm(T11);
-        const float Cp = T00.x * T10.x + T00.y * T10.y + T01.x * T11.x + T01.y * T11.y;
-        const float s1 = cnorm(S1), s2 = cnorm(S2), hd = 0.5f * (Pp - Qp);
-        const float rho = sqrtf(hd * hd + Cp * Cp), den = (s1 + s2) * 0.5f * (Pp + Qp);
-        const float beta = den > 0.f ? fminf(fmaxf(M::div((s2 - s1) * rho, den), -1.f), 1.f) : 0.f;
-        const float irho = rho > 0.f ? M::rcp(rho) : 0.f;  // (cos, sin) of 2 phi0 = (hd, Cp) / rho
-        const float phi = sample_phi<FAST>(u01(r.z), beta, Cp * irho, hd * irho);
-        float sph, cph;
-        if (FAST) __sincosf(phi, &sph, &cph); else sincosf(phi, &sph, &cph);
-        // frame: e1 = cos e_par + sin e_perp, e2 = -sin e_par + cos e_perp
-        const float qx = py * uz - pz * uy, qy = pz * ux - px * uz, qz = px * uy - py * ux;  // e_par
-        const float e1x = cph * qx + sph * px, e1y = cph * qy + sph * py, e1z = cph * qz + sph * pz;
-        float e2x = -sph * qx + cph * px, e2y = -sph * qy + cph * py, e2z = -sph * qz + cph * pz;
-        float nux = cth * ux + sth * e1x, nuy = cth * uy + sth * e1y, nuz = cth * uz + sth * e1z;
-        const float ru = rsqrtf(nux * nux + nuy * nuy + nuz * nuz);
-        nux *= ru;
-        nuy *= ru;
-        nuz *= ru;
-        const float dp = e2x * nux + e2y * nuy + e2z * nuz;
-        e2x -= dp * nux;
-        e2y -= dp * nuy;
-        e2z -= dp * nuz;
-        const float rp = rsqrtf(e2x * e2x + e2y * e2y + e2z * e2z);
-        ux = nux;
-        uy = nuy;
-        uz = nuz;
-        px = e2x * rp;
-        py = e2y * rp;
-        pz = e2z * rp;
-        // Jones: rows of R(phi) T, then diag(S2, S1)
-        const float2 b00 = make_float2(cph * T00.x + sph * T10.x, cph * T00.y + sph * T10.y);
-        const float2 b01 = make_float2(cph * T01.x + sph * T11.x, cph * T01.y + sph * T11.y);
-        const float2 b10 = make_float2(-sph * T00.x + cph * T10.x, -sph * T00.y + cph * T10.y);
-        const float2 b11 = make_float2(-sph * T01.x + cph * T11.x, -sph * T01.y + cph * T11.y);
-        T00 = cmul(S2, b00);
-        T01 = cmul(S2, b01);
-        T10 = cmul(S1, b10);
-        T11 = cmul(S1, b11);
-        const float fn = cnorm(T00) + cnorm(T01) + cnorm(T10) + cnorm(T11);
-        const float sc = fn > 0.f ? (FAST ? 1.41421356f * rsqrtf(fn) : sqrtf(2.f / fn)) : 0.f;
-        T00 = make_float2(T00.x * sc, T00.y * sc);
-        T01 = make_float2(T01.x * sc, T01.y * sc);
-        T10 = make_float2(T10.x * sc, T10.y * sc);
-        T11 = make_float2(T11.x * sc, T11.y * sc);
-        if (med == 0) {
-          if (nsc == 0) {
-            fx = x;
-            fy = y;
-          }
-          lx = x;
-          ly = y;
-        }
-        ++nsc;
-      }
-      if (w < kEfRoulette) {
-        const uint4 a = philox4x32_10(make_uint4(c0, c1, hop | 0x40000000u, kEfTag), P.k0, k1);
-        if (u01(a.y) <= kEfChance)
-          w *= 1.f / kEfChance;
-        else
-          alive = false;
-      }
-      if (++hop >= P.step_cap) {
-        atomicOr(P.flags, (unsigned int)NMC_DEVFLAG_STEPCAP);
-        alive = false;
-      }
+  // the random part of a scattering, from its uniform alone: the angle and the
+  // amplitudes of medium m's table there
+  auto amplitudes = [&](int m, float uth, float& sth, float& cth, float2& S1, float2& S2) {
+    const EfMedium& Md = P.med[m];
+    const float* cdf = s_cdf + Md.cdf_off;
+    const unsigned int* gd = s_guide + m * (kEfGuide + 1);
+    const int gk = min((int)(uth * kEfGuide), kEfGuide - 1);
+    int a0 = (int)gd[gk], a1 = min((int)gd[gk + 1] + 1, P.n_angles - 1);
+    while (a1 - a0 > 1) {
+      const int mid = (a0 + a1) >> 1;
+      if (cdf[mid] <= uth) a0 = mid; else a1 = mid;
     }
+    const float q0 = cdf[a0], q1 = cdf[a1];
+    const float fr = q1 > q0 ? fminf(fmaxf(M::div(uth - q0, q1 - q0), 0.f), 1.f) : 0.5f;
+    const float th = ((float)a0 + fr) * P.dtheta;
+    if (FAST) __sincosf(th, &sth, &cth); else sincosf(th, &sth, &cth);
+    const float4 A0 = __ldg(Md.S + a0), A1 = __ldg(Md.S + a1);
+    S1 = make_float2(fmaf(fr, A1.x - A0.x, A0.x), fmaf(fr, A1.y - A0.y, A0.y));
+    S2 = make_float2(fmaf(fr, A1.z - A0.z, A0.z), fmaf(fr, A1.w - A0.w, A0.w));
+  };
+  // moves by s; false when the photon left through the surface
+  auto move = [&](float s) {
+    if (uz < 0.f && z + s * uz < 0.f) {  // reaches the surface
+      const float d = -z / uz;
+      x = fmaf(d, ux, x);
+      y = fmaf(d, uy, y);
+      z = 0.f;
+      path.add(d);
+      float uzt;
+      const float rsp = rfresnel(P.n_medium, P.n_outside, -uz, &uzt);
+      const uint4 a = philox4x32_10(make_uint4(c0, c1, hop | 0x40000000u, kEfTag), P.k0, k1);
+      if (u01(a.x) > rsp) return false;
+      // mirrored; -M e_perp keeps the frame right-handed, so the perp row flips
+      uz = -uz;
+      px = -px;
+      py = -py;
+      T10 = make_float2(-T10.x, -T10.y);
+      T11 = make_float2(-T11.x, -T11.y);
+      const float rest = s - d;
+      x = fmaf(rest, ux, x);
+      y = fmaf(rest, uy, y);
+      z = rest * uz;
+      path.add(rest);
+    } else {
+      x = fmaf(s, ux, x);
+      y = fmaf(s, uy, y);
+      z = fmaf(s, uz, z);
+      path.add(s);
+    }
+    return true;
+  };
+  auto convert = [&](float uy_, float uz_) {  // Raman conversion
+    med = 1;
+    atomicAdd(&sm[NMC_EF_RAMAN_N], 1.0);
+    if (P.depth) {
+      const int b = (int)(z * P.depth_inv);
+      if (b >= 0 && b < P.depth_bins) atomicAdd(P.depth + (size_t)set * P.depth_bins + b, (double)w);
+    }
+    const float ct = 2.f * uy_ - 1.f, st = sqrtf(fmaxf(0.f, 1.f - ct * ct));
+    float sp, cp;
+    M::sincos2pi(uz_, &sp, &cp);
+    ux = st * cp;
+    uy = st * sp;
+    uz = ct;
+    perp_of(ux, uy, uz, px, py, pz);
+    T00 = make_float2(1.f, 0.f);
+    T01 = make_float2(0.f, 0.f);
+    T10 = make_float2(0.f, 0.f);
+    T11 = make_float2(1.f, 0.f);
+  };
+  // a b + c d: the grades fuse different products there
+  auto turn = [](float a, float b, float c, float d) { return FAST ? dot2(c, d, a, b) : dot2(a, b, c, d); };
+  auto scatter = [&](float sth, float cth, float2 S1, float2 S2, float uphi) {
+    // azimuth from the field: p ∝ 1 + beta cos(2 phi - 2 phi0)
+    const float Pp = norm2(T00) + norm2(T01), Qp = norm2(T10) + norm2(T11);
+    const float Cp = __fmaf_rn(T01.y, T11.y, __fmaf_rn(T01.x, T11.x, dot2(T00.x, T10.x, T00.y, T10.y)));
+    const float s1 = norm2(S1), s2 = norm2(S2), hd = 0.5f * (Pp - Qp);
+    const float rho = sqrtf(dot2(Cp, Cp, hd, hd)), den = (s1 + s2) * 0.5f * (Pp + Qp);
+    const float beta = den > 0.f ? fminf(fmaxf(M::div((s2 - s1) * rho, den), -1.f), 1.f) : 0.f;
+    const float irho = rho > 0.f ? M::rcp(rho) : 0.f;  // (cos, sin) of 2 phi0 = (hd, Cp) / rho
+    const float phi = sample_phi<FAST>(uphi, beta, Cp * irho, hd * irho);
+    float sph, cph;
+    if (FAST) __sincosf(phi, &sph, &cph); else sincosf(phi, &sph, &cph);
+    // frame: e1 = cos e_par + sin e_perp, e2 = -sin e_par + cos e_perp
+    const float qx = det2(py, uz, pz, uy), qy = det2(pz, ux, px, uz), qz = det2(px, uy, py, ux);  // e_par
+    const float e1x = turn(cph, qx, sph, px), e1y = turn(cph, qy, sph, py), e1z = turn(cph, qz, sph, pz);
+    float e2x = dot2(cph, px, -sph, qx), e2y = dot2(cph, py, -sph, qy), e2z = dot2(cph, pz, -sph, qz);
+    float nux = dot2(cth, ux, sth, e1x), nuy = dot2(cth, uy, sth, e1y), nuz = dot2(cth, uz, sth, e1z);
+    const float ru = rsqrtf(dot3(nux, nuy, nuz, nux, nuy, nuz));
+    nux *= ru;
+    nuy *= ru;
+    nuz *= ru;
+    const float dp = dot3(e2x, e2y, e2z, nux, nuy, nuz);
+    e2x = __fmaf_rn(-dp, nux, e2x);
+    e2y = __fmaf_rn(-dp, nuy, e2y);
+    e2z = __fmaf_rn(-dp, nuz, e2z);
+    const float rp = rsqrtf(dot3(e2x, e2y, e2z, e2x, e2y, e2z));
+    ux = nux;
+    uy = nuy;
+    uz = nuz;
+    px = e2x * rp;
+    py = e2y * rp;
+    pz = e2z * rp;
+    // Jones: rows of R(phi) T, then diag(S2, S1)
+    const float2 b00 = make_float2(turn(cph, T00.x, sph, T10.x), turn(cph, T00.y, sph, T10.y));
+    const float2 b01 = make_float2(turn(cph, T01.x, sph, T11.x), turn(cph, T01.y, sph, T11.y));
+    const float2 b10 = make_float2(dot2(cph, T10.x, -sph, T00.x), dot2(cph, T10.y, -sph, T00.y));
+    const float2 b11 = make_float2(dot2(cph, T11.x, -sph, T01.x), dot2(cph, T11.y, -sph, T01.y));
+    T00 = cmul_fused(S2, b00);
+    T01 = cmul_fused(S2, b01);
+    T10 = cmul_fused(S1, b10);
+    T11 = cmul_fused(S1, b11);
+    const float fn = norm2(T00) + norm2(T01) + norm2(T10) + norm2(T11);
+    const float sc = fn > 0.f ? (FAST ? 1.41421356f * rsqrtf(fn) : sqrtf(2.f / fn)) : 0.f;
+    T00 = make_float2(T00.x * sc, T00.y * sc);
+    T01 = make_float2(T01.x * sc, T01.y * sc);
+    T10 = make_float2(T10.x * sc, T10.y * sc);
+    T11 = make_float2(T11.x * sc, T11.y * sc);
+    if (med == 0) {
+      if (nsc == 0) {
+        fx = x;
+        fy = y;
+      }
+      lx = x;
+      ly = y;
+    }
+    ++nsc;
+  };
+  auto roulette = [&]() {
+    if (w < kEfRoulette) {
+      const uint4 a = philox4x32_10(make_uint4(c0, c1, hop | 0x40000000u, kEfTag), P.k0, k1);
+      if (u01(a.y) <= kEfChance)
+        w *= 1.f / kEfChance;
+      else
+        alive = false;
+    }
+    if (++hop >= P.step_cap) {
+      atomicOr(P.flags, (unsigned int)NMC_DEVFLAG_STEPCAP);
+      alive = false;
+    }
+  };
+  auto finish = [&]() {
     atomicAdd(&sm[NMC_EF_SCATTERS], (double)nsc);
-    if (!escaped) continue;
+    if (!escaped) return;
 
     // ---- detection: lab analysers x, y projected perpendicular to the exit direction
     const float qx = py * uz - pz * uy, qy = pz * ux - px * uz, qz = px * uy - py * ux;  // e_par
@@ -395,7 +399,7 @@ __global__ void __launch_bounds__(256) efield_kernel(const EfParams P) {
       A[a][0] = make_float2(T00.x * cpar + T10.x * cperp, T00.y * cpar + T10.y * cperp);
       A[a][1] = make_float2(T01.x * cpar + T11.x * cperp, T01.y * cpar + T11.y * cperp);
     }
-    const float ex = S.ex, ey = S.ey;
+    const float ex = P.sets[set].ex, ey = P.sets[set].ey;
     // fields of input e in the analysers x, y; co = e.(A e), cross = e_perp.(A e)
     const float2 Fx = make_float2(A[0][0].x * ex + A[0][1].x * ey, A[0][0].y * ex + A[0][1].y * ey);
     const float2 Fy = make_float2(A[1][0].x * ex + A[1][1].x * ey, A[1][0].y * ex + A[1][1].y * ey);
@@ -406,7 +410,7 @@ __global__ void __launch_bounds__(256) efield_kernel(const EfParams P) {
       atomicAdd(&sm[NMC_EF_RAMAN_RD], (double)w);
       atomicAdd(&sm[NMC_EF_RAMAN_CO], (double)Ico);
       atomicAdd(&sm[NMC_EF_RAMAN_CROSS], (double)Icr);
-      continue;
+      return;
     }
     atomicAdd(&sm[NMC_EF_RD], (double)w);
     atomicAdd(&sm[NMC_EF_RD2], (double)w * (double)w);
@@ -471,6 +475,114 @@ __global__ void __launch_bounds__(256) efield_kernel(const EfParams P) {
             P.spk[((size_t)set * P.spk_max + k) * MN + pix] =
                 nmc_speckle{a_co, wrap_pi(ph_path), a_cr, wrap_pi(a_co + ph_path), Ixx, Ixy, w};
         }
+      }
+    }
+  };
+
+  const bool idle = LAT && (threadIdx.x & 31) >= P.lanes;
+  while (!idle) {
+    const unsigned long long g = next_photon(P.work);
+    if (g >= P.total) {
+      if (LAT) atomicAdd(&s_idle[threadIdx.x >> 5], 1);
+      break;
+    }
+    int lo = 0, hi = P.nsets;
+    while (hi - lo > 1) {
+      const int mid = (lo + hi) >> 1;
+      if (__ldg(P.prefix + mid) <= g) lo = mid; else hi = mid;
+    }
+    set = lo;
+    const EfSet& S = P.sets[set];
+    const unsigned long long pid = S.first + (g - __ldg(P.prefix + set));
+    k1 = P.k1 + (uint32_t)set, c0 = (uint32_t)pid, c1 = (uint32_t)(pid >> 32);
+    sm = s_sum + set * NMC_EF_FIELDS;
+    atomicAdd(&sm[NMC_EF_PHOTONS], 1.0);
+    atomicAdd(&sm[NMC_EF_SPECULAR], (double)(1.f - S.w0));
+
+    x = y = z = fx = fy = lx = ly = 0.f;
+    ux = S.ux, uy = S.uy, uz = S.uz, px = S.px, py = S.py, pz = S.pz;
+    T00 = S.t[0], T01 = S.t[1], T10 = S.t[2], T11 = S.t[3];
+    w = S.w0;
+    path = PathSum();
+    med = 0;
+    nsc = 0;
+    hop = 0;
+    alive = true;
+    escaped = false;
+    bool leave = false;
+    while (alive) {
+      const uint4 r = philox4x32_10(make_uint4(c0, c1, hop, kEfTag), P.k0, k1);
+      const EfMedium& Md = P.med[med];
+      if (!move(M::neglog(u01(r.x)) * Md.inv_mut)) {
+        escaped = true;
+        break;
+      }
+      w *= Md.surv;
+      if (med == 0 && u01(r.w) < Md.p_raman) {
+        convert(u01(r.y), u01(r.z));
+      } else {
+        float sth, cth;
+        float2 S1, S2;
+        amplitudes(med, u01(r.y), sth, cth, S1, S2);
+        scatter(sth, cth, S1, S2, u01(r.z));
+      }
+      roulette();
+      if (LAT && hop % kThinLook == 0 && alive) {  // go on thin: the queue is empty and few lanes have a photon
+        const int none = *(volatile int*)&s_idle[threadIdx.x >> 5];
+        leave = (int)P.lanes - none <= kThinPhotons && (none > 0 || *(volatile unsigned long long*)P.work >= P.total);
+        if (leave) break;
+      }
+    }
+    if (LAT && leave) {
+      have = true;
+      break;
+    }
+    finish();
+    alive = false;
+  }
+
+  if constexpr (LAT) {
+    // the lanes without a photon compute the random part of the coming hops
+    const unsigned int lane = threadIdx.x & 31, all = 0xFFFFFFFFu;
+    alive = have;
+    unsigned int mask;
+    while ((mask = __ballot_sync(all, alive)) != 0) {
+      const int n = __popc(mask), per = 32 / n;  // photons, and hops of each in this pass
+      const int first = __popc(mask & ((1u << lane) - 1u)) * per;  // my photon's first record
+      const int q = (int)lane / per, src = (int)__fns(mask, 0, min(q, n - 1) + 1);
+      const uint32_t p0 = __shfl_sync(all, c0, src), p1 = __shfl_sync(all, c1, src), pk = __shfl_sync(all, k1, src);
+      const uint32_t h = __shfl_sync(all, hop, src) + (lane - q * per);
+      const int m = __shfl_sync(all, med, src);
+      const uint4 b = philox4x32_10(make_uint4(p0, p1, h, kEfTag), P.k0, pk);
+      const float r_s = M::neglog(u01(b.x)) * P.med[m].inv_mut;
+      float r_sth, r_cth;
+      float2 r_S1, r_S2;
+      amplitudes(m, u01(b.y), r_sth, r_cth, r_S1, r_S2);
+      bool stale = false;  // converted in this pass: the records are of the other medium
+      for (int o = 0; o < per; ++o) {
+        const int k = first + o;
+        const float s = __shfl_sync(all, r_s, k), sth = __shfl_sync(all, r_sth, k), cth = __shfl_sync(all, r_cth, k);
+        const float2 S1 = make_float2(__shfl_sync(all, r_S1.x, k), __shfl_sync(all, r_S1.y, k));
+        const float2 S2 = make_float2(__shfl_sync(all, r_S2.x, k), __shfl_sync(all, r_S2.y, k));
+        const float uphi = u01(__shfl_sync(all, b.z, k)), uram = u01(__shfl_sync(all, b.w, k));
+        if (!alive || stale) continue;
+        if (!move(s)) {
+          escaped = true;
+          alive = false;
+          continue;
+        }
+        w *= P.med[med].surv;
+        if (med == 0 && uram < P.med[0].p_raman) {
+          convert(u01(philox4x32_10(make_uint4(c0, c1, hop, kEfTag), P.k0, k1).y), uphi);
+          stale = true;
+        } else {
+          scatter(sth, cth, S1, S2, uphi);
+        }
+        roulette();
+      }
+      if (have && !alive) {
+        finish();
+        have = false;
       }
     }
   }
@@ -917,18 +1029,27 @@ extern "C" nmc_status nmc_efield_run(int32_t device, const nmc_efield_config* cf
   P.spk_max = spk ? c.speckle_max : 0u;
 
   const bool fast = !(c.flags & NMC_FLAG_PRECISE_MATH);
-  const void* f = fast ? (const void*)efield_kernel<true> : (const void*)efield_kernel<false>;
+  int nsm = 0;
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device);
+  const unsigned long long warps = (unsigned long long)nsm * kLatBlocks * (kLatBlock / 32);
+  // Up to 32 photons per lane of the latency variant it is the faster one (8
+  // settings, about 5,300 scatterings per photon and up to 95,000: 800 photons
+  // take 59 against 88 ms, 8e4 127 / 169, 1e6 205 / 291, 2e6 307 / 342, 4e6
+  // 531 / 513 ms).
+  const bool lat = P.total <= warps * 32 * 32;
+  P.lanes = (unsigned int)std::max<unsigned long long>(1, std::min<unsigned long long>(32, (P.total + warps - 1) / warps));
+  const void* f = lat ? (fast ? (const void*)efield_kernel<true, true> : (const void*)efield_kernel<false, true>)
+                      : (fast ? (const void*)efield_kernel<true, false> : (const void*)efield_kernel<false, false>);
   const size_t smem = sizeof(float) * 2 * n;
   if (smem > 48 * 1024 && cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
                               cudaSuccess)
     return done(NMC_EINVAL);
-  int per_sm = 0, nsm = 0;
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device);
+  int per_sm = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f, 256, smem) != cudaSuccess || per_sm < 1)
     return done(NMC_EDEVICE);
-  const unsigned long long grid =
-      std::max<unsigned long long>(1, std::min<unsigned long long>((unsigned long long)nsm * per_sm,
-                                                                   (P.total + 255) / 256));
+  if (lat) per_sm = std::min(per_sm, kLatBlocks);
+  const unsigned long long grid = std::max<unsigned long long>(
+      1, std::min<unsigned long long>((unsigned long long)nsm * per_sm, lat ? P.total : (P.total + 255) / 256));
   void* args[] = {(void*)&P};
   if (P.total > 0 && cudaLaunchKernel(f, dim3((unsigned)grid), dim3(256), args, smem, st) != cudaSuccess)
     return done(NMC_EDEVICE);
