@@ -388,6 +388,31 @@ struct AdjArgs {
 
 nmc_status fold(nmc_handle* h);
 
+// The launch shape of a voxel run whose caller left it to the library, from
+// its queue items (photons, or runs of photons).  A voxel sub-step takes a lone
+// photon 0.49 us, a photon in a full warp 1.4 us (its 31 neighbours walk other
+// branches) and one of eight full warps on a scheduler 2 us, so:
+//  * up to 5 items per warp of two blocks per SM, each warp takes as few items
+//    as fill them all (blocks of that many threads): 1e3 photons through the
+//    skin-vessel map take 5.9 instead of 10.1 ms, 1e4 8.7 / 10.2;
+//  * while photons per lane are few the tail of long photons outweighs the
+//    throughput that more warps give (4, 6, 8 warps per scheduler: 77, 94,
+//    100%): 1e5 photons take 14.7 / 16.8 / 16.4 ms at 2, 3, 4 blocks per SM,
+//    3e5 20.3 / 20.5 / 23.1, 1e6 48 / 42 / 43; a sweep's sets differ and its
+//    tail is longer: 1.4e6 photons 45-67 / 54-80 / 67-98 ms, 3.5e6 60-82 /
+//    62-93 / 76-113, 7e6 119-144 / 96-123 / 92-136;
+//  * photons that end at the grid's faces (boundaryflag 1) have no such tail.
+struct VoxelShape {
+  int block, per_sm;
+};
+VoxelShape voxel_shape(const nmc_handle* h, uint64_t items, bool sweep) {
+  const uint64_t warps = (uint64_t)h->nsm * 2 * (256 / 32), lanes = warps * 32;
+  if (items <= 5 * warps) return {(int)std::max<uint64_t>(1, (items + warps - 1) / warps), 16};
+  if (h->rp.boundaryflag == 1) return {256, 4};
+  if (sweep) return {256, items <= 26 * lanes ? 2 : items <= 64 * lanes ? 3 : 4};
+  return {256, 2 * items <= 3 * lanes ? 2 : items <= 5 * lanes ? 3 : 4};
+}
+
 nmc_status launch(nmc_handle* h, uint64_t first, uint64_t n, nmc_photon_record* d_recs,
                   float4* d_events, uint32_t k_events, const AdjArgs* adj = nullptr) {
   if (!h->prepared) return fail(h, NMC_ESTATE, "nmc_prepare has not been called");
@@ -466,13 +491,16 @@ nmc_status launch(nmc_handle* h, uint64_t first, uint64_t n, nmc_photon_record* 
         p.dl_next = h->d_dlnext;
       }
     }
-    block = h->ext.block_size > 0 ? h->ext.block_size : 256;
+    const bool own = !trace && h->ext.block_size <= 0 && h->ext.blocks_per_sm <= 0;
+    const VoxelShape shape = voxel_shape(h, (n + p.per_fetch - 1) / p.per_fetch, false);
+    block = own ? shape.block : h->ext.block_size > 0 ? h->ext.block_size : 256;
     const bool tt = h->sim == NMC_SIM_MCXYZ_TT;
     const int mode = !adj ? nmc::kVoxel : adj->pass == 0 ? nmc::kRecord : adj->pass == 2 ? nmc::kScore : nmc::kAdjoint;
     if (h->voxel_mode)
       NMC_CUDA(h, nmc::mcxyz_voxel_occupancy(mode, trace, block, &per_sm));
     else
       NMC_CUDA(h, nmc::mcxyz_occupancy(tt, trace, block, &per_sm));
+    if (own) per_sm = std::min(per_sm, shape.per_sm);
     if (h->ext.blocks_per_sm > 0) per_sm = std::min(per_sm, (int)h->ext.blocks_per_sm);
     if (per_sm < 1) return fail(h, NMC_EDEVICE, "mcxyz kernel does not fit on an SM with this block size");
     uint64_t grid = (uint64_t)h->nsm * per_sm;
@@ -1349,10 +1377,13 @@ nmc_status nmc_run_sweep_tissues(nmc_handle* h, const nmc_tissue_params* tables,
       cudaMemsetAsync(&h->d_sums->work, 0, sizeof(unsigned long long), h->stream) != cudaSuccess)
     return fail(h, NMC_EDEVICE, "sweep buffer set-up");
   const bool tt = h->sim == NMC_SIM_MCXYZ_TT;
-  const int block = h->ext.block_size > 0 ? h->ext.block_size : 256;
+  const bool own = h->ext.block_size <= 0 && h->ext.blocks_per_sm <= 0;
+  const VoxelShape shape = voxel_shape(h, (p.n + p.per_fetch - 1) / p.per_fetch, true);
+  const int block = own ? shape.block : h->ext.block_size > 0 ? h->ext.block_size : 256;
   int per_sm = 0;
   if (nmc::mcxyz_sweep_occupancy(tt, block, &per_sm) != cudaSuccess || per_sm < 1)
     return fail(h, NMC_EDEVICE, "sweep kernel does not fit on an SM");
+  if (own) per_sm = std::min(per_sm, shape.per_sm);
   if (h->ext.blocks_per_sm > 0) per_sm = std::min(per_sm, (int)h->ext.blocks_per_sm);
   uint64_t grid = (uint64_t)h->nsm * per_sm;
   grid = std::max<uint64_t>(1, std::min<uint64_t>(grid, (p.n + block - 1) / block));
