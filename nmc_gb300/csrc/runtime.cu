@@ -18,6 +18,7 @@
 #include <cstring>
 #include <new>
 #include <string>
+#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -348,7 +349,12 @@ nmc_status wait_event(nmc_handle* h, cudaEvent_t ev) {
     if (q != cudaErrorNotReady) return cuda_fail(h, q, "kernel execution");
     const double el = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
     if (el > limit) return fail(h, NMC_ETIMEOUT, "device work did not finish within timeout_s");
-    std::this_thread::sleep_for(std::chrono::microseconds(el < 0.01 ? 20 : 500));
+    // the first millisecond awake (a sleep takes 70 us or more to return),
+    // then naps of half a percent of the time waited
+    if (el < 0.001)
+      std::this_thread::yield();
+    else
+      std::this_thread::sleep_for(std::chrono::microseconds(std::min(500, std::max(20, (int)(el * 5000.0)))));
   }
 }
 
@@ -1067,6 +1073,29 @@ nmc_status nmc_get_tally_f64(nmc_handle* h, int32_t which, double* out, size_t n
   return NMC_OK;
 }
 
+// dst[i] += src[i]; a 200^3 fluence map is 32 MB on each side, which one core
+// adds in 4 to 8 ms (the caller's fresh pages are first touched here), so large
+// arrays are shared among up to 8 threads.
+static void add_to(float* dst, const float* src, size_t n) {
+  const auto part = [=](size_t a, size_t b) {
+    for (size_t i = a; i < b; ++i) dst[i] += src[i];
+  };
+  constexpr size_t kPart = 1 << 18;  // 1 MB, about 0.2 ms of work
+  const size_t want = std::min<size_t>({8, n / kPart, std::max(1u, std::thread::hardware_concurrency())});
+  const size_t step = want > 1 ? (n / want + 15) & ~(size_t)15 : n;
+  std::vector<std::thread> others;
+  size_t done = 0;
+  if (want > 1) {
+    others.reserve(want - 1);
+    try {
+      for (; others.size() + 1 < want; done += step) others.emplace_back(part, done, done + step);
+    } catch (const std::system_error&) {  // no more threads: this one does the rest
+    }
+  }
+  part(done, n);
+  for (std::thread& t : others) t.join();
+}
+
 nmc_status nmc_get_compute_results(nmc_handle* h, float* J, float* F, float* F3D, float* SAE,
                                    float* Rd, float* Rd2D, int32_t* DetPhot2D, float* PolXX,
                                    float* PolXY, float* PolYX, float* PolYY, float* Phase0,
@@ -1111,8 +1140,7 @@ nmc_status nmc_get_compute_results(nmc_handle* h, float* J, float* F, float* F3D
       const unsigned int* c = reinterpret_cast<const unsigned int*>(src);
       for (size_t i = 0; i < n; ++i) DetPhot2D[i] += (int32_t)c[i];
     } else {
-      float* d = dst[k];
-      for (size_t i = 0; i < n; ++i) d[i] += src[i];
+      add_to(dst[k], src, n);
     }
   }
   return NMC_OK;
