@@ -90,3 +90,26 @@ def test_field(gpu, oracle, photons):
         assert np.all(np.abs(g[k] - o[k]) <= 1e-3 * (o["Rd"] + o["raman_Rd"]) + 1e-3), k
     for k in ("raman_n", "scatters"):
         assert np.all(np.abs(g[k] - o[k]) <= 2e-3 * o[k] + 2), k
+
+
+@pytest.mark.parametrize("n", [1, 2432, 2433, 4865, 9729, 12_160, 12_161, 116_737, 389_121])
+@pytest.mark.parametrize("sim,boundary,rng", [(abi.SIM_MCXYZ, 2, abi.RNG_PHILOX), (abi.SIM_MCXYZ, 1, abi.RNG_TAUS_REF),
+                                              (abi.SIM_MCXYZ_TT, 0, abi.RNG_PHILOX)])
+def test_voxel_launch_shapes(gpu, sim, boundary, rng, n):
+    # one photon per warp, a few (blocks of 1 to 5 threads), 2, 3 and 4 blocks
+    # per SM: the same tallies as blocks of 256 that fill the GPU
+    rp, tp, v = cases.modes_medium(boundaryflag=boundary, mckernelflag=sim)
+    if sim == abi.SIM_MCXYZ_TT:
+        tp = abi.tissue_params(mua=[0.0001, 1.0, 5.0], mus=[1.0, 80.0, 120.0], g=[1.0, 0.85, 0.9], gf=[0.9] * 3, af=[0.5] * 3,
+                               gb=[0.3] * 3, ab=[0.5] * 3, cc=[0.9] * 3)
+    got = []
+    for block in (0, 256):
+        with gpu.Engine(sim, 0, abi.ext_defaults(seed=5, rng=rng, block_size=block)) as e:
+            e.prepare_data(rp, tp, v)
+            e.run(7, n)
+            one = (e.summary(), e.get_compute_results())
+            sweep = e.run_sweep_tissues([tp, tp], [n, n // 3]) if rng == abi.RNG_PHILOX else {}
+        got.append((one, sweep))
+    _same(got[0][0], got[1][0])
+    for k in got[0][1]:
+        np.testing.assert_allclose(got[0][1][k], got[1][1][k], rtol=1e-12 if k in ("E2", "Rd_se") else 0, err_msg=k)
