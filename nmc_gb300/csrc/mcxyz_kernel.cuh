@@ -247,7 +247,9 @@ __global__ void __launch_bounds__(256, 4) mcxyz_kernel(const XyzParams P) {
       s_ph[t] = P.phase[t];
     }
   }
-  for (int t = threadIdx.x; t < 5; t += blockDim.x) s_tot[t] = 0ull;  // (blocks may have fewer threads)
+  if (threadIdx.x < 5) s_tot[threadIdx.x] = 0ull;
+  if (blockDim.x < 5 && threadIdx.x == 0)  // fewer threads than sums
+    for (int t = blockDim.x; t < 5; ++t) s_tot[t] = 0ull;
   if (threadIdx.x == 0) s_rd2 = 0.0;
   __syncthreads();
 
@@ -702,15 +704,17 @@ __global__ void __launch_bounds__(256, 4) mcxyz_kernel(const XyzParams P) {
 
   if (REC && dl_chunk < kDeadChunk) P.dl_fill[dl_chunk] = dl_pos;
   __syncthreads();
-  for (int t = threadIdx.x; t < 5; t += blockDim.x) {
-    if (!s_tot[t]) continue;
-    unsigned long long* dst = t == 0   ? &P.sums->photons
-                              : t == 1 ? &P.sums->substeps
-                              : t == 2 ? &P.sums->scatters
-                              : t == 3 ? &P.sums->A
-                                       : &P.sums->rd;
-    atomicAdd(dst, s_tot[t]);
+  if (threadIdx.x < 5 && s_tot[threadIdx.x]) {
+    unsigned long long* dst = threadIdx.x == 0   ? &P.sums->photons
+                              : threadIdx.x == 1 ? &P.sums->substeps
+                              : threadIdx.x == 2 ? &P.sums->scatters
+                              : threadIdx.x == 3 ? &P.sums->A
+                                                 : &P.sums->rd;
+    atomicAdd(dst, s_tot[threadIdx.x]);
   }
+  if (blockDim.x < 5 && threadIdx.x == 0)
+    for (int t = blockDim.x; t < 5; ++t)
+      atomicAdd(t == 1 ? &P.sums->substeps : t == 2 ? &P.sums->scatters : t == 3 ? &P.sums->A : &P.sums->rd, s_tot[t]);
   if (threadIdx.x == 0 && s_rd2 != 0.0) atomicAdd(&P.sums->rd_sumsq, s_rd2);
 }
 
