@@ -534,7 +534,12 @@ nmc_status layered_impl(int32_t device, const nmc_layered_config* cfg, const nmc
   int per_sm = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f, 256, smem) != cudaSuccess || per_sm < 1)
     return done(NMC_EDEVICE);
-  if (lat) per_sm = std::min(per_sm, kLatBlocks);
+  // Up to eight photons per lane of two blocks per SM, the throughput variant
+  // also runs two: the tail of long photons is most of the run, and among
+  // fewer warps a step takes less time (three-layer skin at 2 / 4 blocks: 3.2e5
+  // photons 13.6 / 16 ms, 5e5 14.8 / 16.3, 6e5 15.8 / 17.1; adjoint 6e5 20.0 /
+  // 21.4; reference streams 1e5 8.8 / 10.5; 1e6 21.2 / 20.3).
+  if (photons <= warps * 256) per_sm = std::min(per_sm, kLatBlocks);
   const unsigned long long grid = std::max<unsigned long long>(
       1, std::min<unsigned long long>((unsigned long long)nsm * per_sm, lat ? photons : (photons + 255) / 256));
   void* args[] = {(void*)&P};
