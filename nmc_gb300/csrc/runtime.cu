@@ -1086,10 +1086,10 @@ static void add_to(float* dst, const float* src, size_t n) {
   std::vector<std::thread> others;
   size_t done = 0;
   if (want > 1) {
-    others.reserve(want - 1);
     try {
+      others.reserve(want - 1);
       for (; others.size() + 1 < want; done += step) others.emplace_back(part, done, done + step);
-    } catch (const std::system_error&) {  // no more threads: this one does the rest
+    } catch (const std::exception&) {  // no more threads or memory: this one does the rest
     }
   }
   part(done, n);
