@@ -16,9 +16,9 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <exception>
 #include <new>
 #include <string>
-#include <system_error>
 #include <thread>
 #include <vector>
 
