@@ -293,7 +293,9 @@ cudaError_t sweep_prepare(const SweepParams& p, const void** f, size_t* sh) {
   else
     *f = p.fast ? pick<true, false>(p.phase_kind) : pick<false, false>(p.phase_kind);
   *sh = sweep_smem_bytes(p.nsets);
-  if (*sh > 48 * 1024) return cudaFuncSetAttribute(*f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)*sh);
+  // a block's static shared memory counts against the 48 KB it has without
+  // this; 1024 sets alone take all of it
+  if (*sh > 32 * 1024) return cudaFuncSetAttribute(*f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)*sh);
   return cudaSuccess;
 }
 
