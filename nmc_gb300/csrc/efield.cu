@@ -1036,12 +1036,25 @@ extern "C" nmc_status nmc_efield_run(int32_t device, const nmc_efield_config* cf
   // settings, about 5,300 scatterings per photon and up to 95,000: 800 photons
   // take 59 against 88 ms, 8e4 127 / 169, 1e6 205 / 291, 2e6 307 / 342, 4e6
   // 531 / 513 ms).
-  const bool lat = P.total <= warps * 32 * 32;
-  P.lanes = (unsigned int)std::max<unsigned long long>(1, std::min<unsigned long long>(32, (P.total + warps - 1) / warps));
-  const void* f = lat ? (fast ? (const void*)efield_kernel<true, true> : (const void*)efield_kernel<false, true>)
-                      : (fast ? (const void*)efield_kernel<true, false> : (const void*)efield_kernel<false, false>);
+  // The tables (8 bytes per angle) share a block's memory with the kernel's
+  // static arrays; the latency variant has 32 bytes more of them, so the last
+  // sizes that fit a block at all (27,003 to 27,006 angles) take the other one.
   const size_t smem = sizeof(float) * 2 * n;
-  if (smem > 48 * 1024 && cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
+  int max_smem = 0;
+  cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
+  auto kernel = [&](bool l) {
+    return l ? (fast ? (const void*)efield_kernel<true, true> : (const void*)efield_kernel<false, true>)
+             : (fast ? (const void*)efield_kernel<true, false> : (const void*)efield_kernel<false, false>);
+  };
+  auto fits = [&](const void* k) {
+    cudaFuncAttributes a{};
+    return cudaFuncGetAttributes(&a, k) == cudaSuccess && a.sharedSizeBytes + smem <= (size_t)max_smem;
+  };
+  const bool lat = P.total <= warps * 32 * 32 && fits(kernel(true));
+  P.lanes = (unsigned int)std::max<unsigned long long>(1, std::min<unsigned long long>(32, (P.total + warps - 1) / warps));
+  const void* f = kernel(lat);
+  // above 48 KB together with the static arrays a block must ask for it
+  if (smem > 16 * 1024 && cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
                               cudaSuccess)
     return done(NMC_EINVAL);
   int per_sm = 0;

@@ -25,3 +25,17 @@ def test_sweep_of_the_most_sets(gpu, phase, n_sets):
     assert np.all(got[0]["photons"] == 20)
     for k in got[0]:
         (np.testing.assert_allclose if k in ("E2", "Rd_se") else np.testing.assert_array_equal)(got[0][k], got[1][k], err_msg=k)
+
+
+@pytest.mark.parametrize("flags", [0, abi.FLAG_PRECISE_MATH])
+@pytest.mark.parametrize("n_angles", [4090, 4091, 4094, 27_002, 27_003, 27_006])
+def test_field_of_the_most_angles(gpu, n_angles, flags):
+    # 4,094 angles are what fits 48 KB beside the static arrays of the kernel
+    # that fills the GPU, 27,006 what fits a block at all
+    from nmc_gb300 import efield
+
+    cfg, _, _, st = cases.cbs_case(n_settings=2, photons=500, mu_raman=0.0)
+    cfg.mua, cfg.n_angles, cfg.flags = 5.0, n_angles, flags
+    g = efield.run(cfg, cases.hg_amplitude_table(0.8, n_angles), st, cone=False, pol_vs_scatt=False, maps=False, raman_depth=False)
+    assert list(g["photons"]) == [500, 500]
+    assert np.all(g["Rd"] > 0) and np.all(g["Rd"] < 500)
