@@ -6,6 +6,7 @@
 
 #include <cstdint>
 
+#include "launch_rules.h"
 #include "nmc_abi.h"
 #include "nmc_device.cuh"
 
@@ -36,29 +37,6 @@ struct AdjEvent {
   float w;              // detected weight
   float pad;
 };
-
-// The latency variant of a kernel runs few photons per lane: kLatBlocks blocks
-// of kLatBlock threads per SM (4 warps per scheduler, up to 128 registers)
-// instead of a full SM, and, when the queue is empty, warps that "go on thin":
-// once at most kThinPhotons of a warp's lanes have a photon, the others
-// compute the random part of the coming hops, which depends on the photon and
-// the hop's number alone.  A photon looks for that every kThinLook scatterings.
-//
-// It pays while the run's work is small against its tail: it shortens a long
-// photon's step by about 0.24 us and takes 1.8 ps longer per step of work
-// (semi-infinite kernels, in scatterings: 1.2 against 1.5 e11 per second), so
-// up to about 1.4e5 times the longest photon's scatterings.
-struct LatencyRule {
-  double work = 0.0, tail = 0.0;
-  // n photons in a medium of these coefficients: about 31 (mu_t / mu_a)^0.56
-  // scatterings each (measured from 100 to 10,000: 407, 1,490 and 5,330 at 101,
-  // 1e3 and 1e4), the longest until its weight reaches the roulette's 1e-4
-  void add(double n, double mua, double mus);
-  bool pays() const { return work < 1.4e5 * tail; }
-};
-constexpr int kLatBlock = 256, kLatBlocks = 2;
-constexpr int kThinPhotons = 8;
-constexpr unsigned int kThinLook = 16;
 
 // Voxel kernels (MCXYZKernel kernels.metal:321-754 and MCXYZKernelTT
 // :757-1118).  Photon positions are kept as an integer voxel-lattice cell

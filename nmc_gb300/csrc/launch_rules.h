@@ -1,0 +1,57 @@
+// launch_rules.h - which variant and launch shape a run takes, from its size
+// and its media.  Host arithmetic only: no CUDA header, no state.
+#pragma once
+
+#include <algorithm>
+#include <cmath>
+#include <cstdint>
+
+namespace nmc {
+
+// The latency variant of a kernel runs few photons per lane: kLatBlocks blocks
+// of kLatBlock threads per SM (4 warps per scheduler, up to 128 registers)
+// instead of a full SM, and, when the queue is empty, warps that "go on thin":
+// once at most kThinPhotons of a warp's lanes have a photon, the others
+// compute the random part of the coming hops, which depends on the photon and
+// the hop's number alone.  A photon looks for that every kThinLook scatterings.
+constexpr int kLatBlock = 256, kLatBlocks = 2;
+constexpr int kThinPhotons = 8;
+constexpr unsigned int kThinLook = 16;
+
+// A run's work, in scatterings, and its tail, the scatterings of its longest
+// photon.  Few resident photons finish the tail sooner, many do more work per
+// second, so each kernel has a ratio of the two up to which fewer pay.
+struct WorkTail {
+  double work = 0.0, tail = 0.0;
+  // n photons in a medium of these coefficients: about 31 (mu_t / mu_a)^0.56
+  // scatterings each (measured from 100 to 10,000: 407, 1,490 and 5,330 at 101,
+  // 1e3 and 1e4), the longest until its weight reaches the roulette's 1e-4
+  void add(double n, double mua, double mus) {
+    const double r = std::min((mua + mus) / std::max(mua, 1e-6), 1e6);
+    work += n * 31.0 * std::pow(r, 0.56);
+    if (n > 0.0) tail = std::max(tail, 9.2 * r);
+  }
+  bool below(double ratio) const { return work < ratio * tail; }
+};
+
+// Lanes of each of `warps` warps that take photons, so that below one item
+// per lane they are spread over all the warps that are really resident.
+inline unsigned int lat_lanes(uint64_t items, uint64_t warps) {
+  return (unsigned int)std::max<uint64_t>(1, std::min<uint64_t>(32, (items + warps - 1) / warps));
+}
+
+// The semi-infinite kernel's latency variant.  Its private F(r,z) can leave
+// room for one block per SM only (bins 118 to 158): the variant then has 8
+// warps per SM where the other kernel has 16, and pays up to a smaller ratio.
+// 128 bins, variant against the other, at photons of (mua, mus): (1, 100) 1e4
+// 0.59 / 0.96 ms, 7e4 0.89 / 0.98, 1e5 1.10 / 1.00, 3e5 2.54 / 1.94; (10, 100)
+// 4e4 0.13 / 0.15, 1e5 0.26 / 0.18; (0.2, 300) 2.5e5 13.0 / 13.2, 1e6 33 / 25;
+// the reference's streams cross at the same ratios.
+inline bool sub_latency_pays(const WorkTail& w, int resident_blocks) {
+  return w.below(resident_blocks >= kLatBlocks ? 1.4e5 : 3.7e4);
+}
+
+// The semi-infinite sweep's latency variant (two blocks are always resident).
+inline bool sweep_latency_pays(const WorkTail& w) { return w.below(1.4e5); }
+
+}  // namespace nmc

@@ -2,7 +2,6 @@
 // the reference's configuration (RunParams / TissueParams,
 // definitions.h:186-218) and the extension knobs.  Derived constants are
 // computed in double and rounded once to float.
-#include <algorithm>
 #include <cmath>
 
 #include "engine.h"
@@ -80,12 +79,6 @@ PhaseConst phase_const(const nmc_tissue_params& tp, int t) {
     p.b.e = (float)(1.0 / (2.0 * gb));
   }
   return p;
-}
-
-void LatencyRule::add(double n, double mua, double mus) {
-  const double r = std::min((mua + mus) / std::max(mua, 1e-6), 1e6);
-  work += n * 31.0 * std::pow(r, 0.56);
-  if (n > 0.0) tail = std::max(tail, 9.2 * r);
 }
 
 RngParams rng_params(const nmc_ext& e, int sim) {

@@ -453,22 +453,22 @@ nmc_status launch(nmc_handle* h, uint64_t first, uint64_t n, nmc_photon_record* 
     p.first = first;
     p.n = n;
     p.trace = tr;
-    block = h->ext.block_size > 0 ? h->ext.block_size : 512;
-    // The latency variant where it pays (mua 1, mus 100: 1e4 photons take 0.58
-    // against 0.90 ms, 1e5 1.01 / 1.58, 3e5 1.71 / 1.82, 1e6 4.44 / 3.82 ms);
-    // below one photon per lane they are spread over all its warps.
-    const uint64_t warps = (uint64_t)h->nsm * nmc::kLatBlocks * (nmc::kLatBlock / 32);
+    // The latency variant where it pays (launch_rules.h): mua 1, mus 100: 1e4
+    // photons take 0.58 against 0.90 ms, 1e5 1.01 / 1.58, 1e6 4.44 / 3.82 ms.
     const uint64_t items = (n + p.per_fetch - 1) / p.per_fetch;
-    nmc::LatencyRule rule;
-    rule.add((double)n, p.mua, p.mus);
-    const bool lat = !trace && h->ext.block_size <= 0 && h->ext.blocks_per_sm <= 0 && rule.pays();
-    if (lat) {
-      block = nmc::kLatBlock;
-      p.lanes = (unsigned int)std::min<uint64_t>(32, (items + warps - 1) / warps);
+    bool lat = false;
+    if (!trace && h->ext.block_size <= 0 && h->ext.blocks_per_sm <= 0) {
+      p.lanes = 1;  // the occupancy of the variant decides first
+      NMC_CUDA(h, nmc::mcsub_occupancy(p, false, nmc::kLatBlock, &per_sm));
+      per_sm = std::min(per_sm, nmc::kLatBlocks);
+      nmc::WorkTail w;
+      w.add((double)n, p.mua, p.mus);
+      lat = per_sm >= 1 && nmc::sub_latency_pays(w, per_sm);
+      p.lanes = lat ? nmc::lat_lanes(items, (uint64_t)h->nsm * per_sm * (nmc::kLatBlock / 32)) : 0;
     }
-    NMC_CUDA(h, nmc::mcsub_occupancy(p, trace, block, &per_sm));
+    block = lat ? nmc::kLatBlock : h->ext.block_size > 0 ? h->ext.block_size : 512;
+    if (!lat) NMC_CUDA(h, nmc::mcsub_occupancy(p, trace, block, &per_sm));
     if (h->ext.blocks_per_sm > 0) per_sm = std::min(per_sm, (int)h->ext.blocks_per_sm);
-    if (lat) per_sm = std::min(per_sm, nmc::kLatBlocks);
     if (per_sm < 1) return fail(h, NMC_EDEVICE, "mcsub kernel does not fit on an SM with this block size");
     uint64_t grid = (uint64_t)h->nsm * per_sm;
     grid = lat ? std::min<uint64_t>(grid, items) : std::min<uint64_t>(grid, (n + block - 1) / block);
@@ -1272,10 +1272,10 @@ nmc_status nmc_run_sweep(nmc_handle* h, const nmc_sweep_set* sets, int32_t n_set
   // The latency variant where it pays: 351 long-lived sets of 200, 1e4 and 2e4
   // photons take 12.4, 28.6 and 45.4 ms, against 20.3, 37.6 and 44.8 ms;
   // short-lived ones of 1e3 photons take 1.4 against 1.5 ms, of 4e3 3.5 / 2.7.
-  nmc::LatencyRule rule;
-  for (int k = 0; k < n_sets; ++k) rule.add((double)sets[k].photons, sets[k].mua, sets[k].mus);
-  const bool lat = h->ext.block_size <= 0 && h->ext.blocks_per_sm <= 0 && rule.pays();
-  if (lat) p.lanes = (unsigned int)std::max<uint64_t>(1, std::min<uint64_t>(32, (p.total + warps - 1) / warps));
+  nmc::WorkTail w;
+  for (int k = 0; k < n_sets; ++k) w.add((double)sets[k].photons, sets[k].mua, sets[k].mus);
+  const bool lat = h->ext.block_size <= 0 && h->ext.blocks_per_sm <= 0 && nmc::sweep_latency_pays(w);
+  if (lat) p.lanes = nmc::lat_lanes(p.total, warps);
   const int block = h->ext.block_size > 0 ? h->ext.block_size : 256;
   int per_sm = 0;
   if (nmc::sweep_occupancy(p, block, &per_sm) != cudaSuccess || per_sm < 1)

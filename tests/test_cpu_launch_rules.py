@@ -1,0 +1,44 @@
+"""The launch rules (nmc_gb300/csrc/launch_rules.h) at media and sizes where both variants were timed on a GB300: the
+rule takes the faster one wherever they differ by more than a tenth."""
+import ctypes as C
+import os
+import subprocess
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+SRC = r"""
+#include "launch_rules.h"
+using namespace nmc;
+static WorkTail one(double n, double mua, double mus) { WorkTail w; w.add(n, mua, mus); return w; }
+extern "C" {
+int sub_lat(double n, double mua, double mus, int blocks) { return sub_latency_pays(one(n, mua, mus), blocks); }
+unsigned lanes(unsigned long long items, unsigned long long warps) { return lat_lanes(items, warps); }
+}
+"""
+
+
+@pytest.fixture(scope="session")
+def rules(tmp_path_factory):
+    d = tmp_path_factory.mktemp("rules")
+    (d / "rules.cpp").write_text(SRC)
+    subprocess.run(["g++", "-O1", "-std=c++17", "-shared", "-fPIC", "-I" + os.path.join(ROOT, "nmc_gb300", "csrc"), str(d / "rules.cpp"),
+                    "-o", str(d / "rules.so")], check=True)
+    lib = C.CDLL(str(d / "rules.so"))
+    lib.sub_lat.argtypes = [C.c_double] * 3 + [C.c_int]
+    lib.lanes.argtypes, lib.lanes.restype = [C.c_ulonglong] * 2, C.c_uint
+    return lib
+
+
+@pytest.mark.parametrize("mua,mus,pays,loses", [(1, 100, 70_000, 150_000), (10, 100, 20_000, 70_000), (1, 20, 20_000, 70_000),
+                                                (0.2, 300, 200_000, 400_000), (0.05, 100, 300_000, 400_000)])
+def test_semi_infinite_with_one_block_per_sm(rules, mua, mus, pays, loses):
+    assert rules.sub_lat(pays, mua, mus, 1) and not rules.sub_lat(loses, mua, mus, 1)
+    assert rules.sub_lat(pays, mua, mus, 2)  # two blocks pay at least as long
+
+
+@pytest.mark.parametrize("items,warps,want", [(1, 1216, 1), (1216, 1216, 1), (1217, 1216, 2), (10_000, 1216, 9), (10_000, 2432, 5),
+                                              (38_912, 1216, 32), (1 << 40, 1216, 32), (0, 1216, 1)])
+def test_every_photon_of_a_small_run_has_a_lane(rules, items, warps, want):
+    assert rules.lanes(items, warps) == want
+    assert items > 32 * warps or want * warps >= items

@@ -39,3 +39,23 @@ def test_field_of_the_most_angles(gpu, n_angles, flags):
     g = efield.run(cfg, cases.hg_amplitude_table(0.8, n_angles), st, cone=False, pol_vs_scatt=False, maps=False, raman_depth=False)
     assert list(g["photons"]) == [500, 500]
     assert np.all(g["Rd"] > 0) and np.all(g["Rd"] < 500)
+
+
+@pytest.mark.parametrize("n", [1, 1217, 10_000, 60_000])
+@pytest.mark.parametrize("rng", [abi.RNG_PHILOX, abi.RNG_TAUS_REF])
+def test_semi_infinite_with_one_block_per_sm(gpu, rng, n):
+    # 128 bins: the private F(r,z) leaves room for one block, whose 8 warps per
+    # SM take all the photons
+    rp, tp, ext = cases.mcsub_case(bins=128, rng=rng, seed=5)
+    got = []
+    for block in (0, 512):
+        ext.block_size = block
+        with gpu.Engine(abi.SIM_MCSUB, 0, ext) as e:
+            e.prepare_data(rp, tp)
+            e.run(0, n)
+            got.append((e.summary(), e.get_compute_results()))
+    assert got[0][0]["photons"] == n
+    for k in ("photons", "substeps", "scatters", "S", "A", "E"):
+        assert got[0][0][k] == got[1][0][k], k
+    for k in got[0][1]:
+        np.testing.assert_array_equal(got[0][1][k], got[1][1][k], err_msg=k)
