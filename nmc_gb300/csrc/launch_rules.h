@@ -46,9 +46,12 @@ inline unsigned int lat_lanes(uint64_t items, uint64_t warps) {
 // 128 bins, variant against the other, at photons of (mua, mus): (1, 100) 1e4
 // 0.59 / 0.96 ms, 7e4 0.89 / 0.98, 1e5 1.10 / 1.00, 3e5 2.54 / 1.94; (10, 100)
 // 4e4 0.13 / 0.15, 1e5 0.26 / 0.18; (0.2, 300) 2.5e5 13.0 / 13.2, 1e6 33 / 25;
-// the reference's streams cross at the same ratios.
+// the reference's streams cross at the same ratios.  With two blocks (101 bins):
+// (1, 100) 2e5 1.29 / 1.48, 2.5e5 1.76 / 1.69, 3e5 1.90 / 1.75; (10, 100) 1e5
+// 0.175 / 0.196, 1.5e5 0.24 / 0.20; (0.05, 100) 1e6 30.1 / 31.3: between 1.0e5
+// and 1.3e5 in each medium.
 inline bool sub_latency_pays(const WorkTail& w, int resident_blocks) {
-  return w.below(resident_blocks >= kLatBlocks ? 1.4e5 : 3.7e4);
+  return w.below(resident_blocks >= kLatBlocks ? 1.2e5 : 3.7e4);
 }
 
 // The semi-infinite sweep's latency variant (two blocks are always resident).

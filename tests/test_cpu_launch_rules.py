@@ -42,3 +42,14 @@ def test_semi_infinite_with_one_block_per_sm(rules, mua, mus, pays, loses):
 def test_every_photon_of_a_small_run_has_a_lane(rules, items, warps, want):
     assert rules.lanes(items, warps) == want
     assert items > 32 * warps or want * warps >= items
+
+
+@pytest.mark.parametrize("mua,mus,pays,loses", [(1, 100, 200_000, 600_000), (10, 100, 100_000, 150_000), (1, 20, 100_000, 150_000),
+                                                (0.2, 300, 600_000, 10_000_000), (0.05, 100, 600_000, 10_000_000)])
+def test_semi_infinite_with_two_blocks_per_sm(rules, mua, mus, pays, loses):
+    assert rules.sub_lat(pays, mua, mus, 2) and not rules.sub_lat(loses, mua, mus, 2)
+
+
+def test_semi_infinite_at_the_crossing(rules):
+    # 1.90 against 1.75 ms
+    assert not rules.sub_lat(300_000, 1.0, 100.0, 2)
