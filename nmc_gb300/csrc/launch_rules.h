@@ -55,6 +55,9 @@ inline bool sub_latency_pays(const WorkTail& w, int resident_blocks) {
 }
 
 // The semi-infinite sweep's latency variant (two blocks are always resident).
-inline bool sweep_latency_pays(const WorkTail& w) { return w.below(1.4e5); }
+// 351 sets of mua in the range given, variant against the other: 0.05-2, 4e3
+// photons each 9.2 / 11.8 ms, 1e4 14.4 / 14.2; 0.5-5, 1e3 1.37 / 1.40, 3e3
+// 2.32 / 2.00, two-term 2e3 1.89 / 1.96, 4e3 3.20 / 2.53; 3-30, 1e3 0.43 / 0.38.
+inline bool sweep_latency_pays(const WorkTail& w) { return w.below(8e4); }
 
 }  // namespace nmc

@@ -1269,9 +1269,7 @@ nmc_status nmc_run_sweep(nmc_handle* h, const nmc_sweep_set* sets, int32_t n_set
       cudaMemsetAsync(p.sums, 0, al(b_sums) + al(b_e2) + al(b_work) + al(b_J), h->stream) != cudaSuccess)
     return fail(h, NMC_EDEVICE, "sweep buffer set-up");
   const uint64_t warps = (uint64_t)h->nsm * nmc::kLatBlocks * (nmc::kLatBlock / 32);
-  // The latency variant where it pays: 351 long-lived sets of 200, 1e4 and 2e4
-  // photons take 12.4, 28.6 and 45.4 ms, against 20.3, 37.6 and 44.8 ms;
-  // short-lived ones of 1e3 photons take 1.4 against 1.5 ms, of 4e3 3.5 / 2.7.
+  // the latency variant where it pays (launch_rules.h)
   nmc::WorkTail w;
   for (int k = 0; k < n_sets; ++k) w.add((double)sets[k].photons, sets[k].mua, sets[k].mus);
   const bool lat = h->ext.block_size <= 0 && h->ext.blocks_per_sm <= 0 && nmc::sweep_latency_pays(w);

@@ -13,6 +13,11 @@ using namespace nmc;
 static WorkTail one(double n, double mua, double mus) { WorkTail w; w.add(n, mua, mus); return w; }
 extern "C" {
 int sub_lat(double n, double mua, double mus, int blocks) { return sub_latency_pays(one(n, mua, mus), blocks); }
+int sweep_lat(int sets, double per, double lo, double hi) {
+  WorkTail w;
+  for (int k = 0; k < sets; ++k) w.add(per, lo + (hi - lo) * k / (sets - 1), 100.0);
+  return sweep_latency_pays(w);
+}
 unsigned lanes(unsigned long long items, unsigned long long warps) { return lat_lanes(items, warps); }
 }
 """
@@ -26,6 +31,7 @@ def rules(tmp_path_factory):
                     "-o", str(d / "rules.so")], check=True)
     lib = C.CDLL(str(d / "rules.so"))
     lib.sub_lat.argtypes = [C.c_double] * 3 + [C.c_int]
+    lib.sweep_lat.argtypes = [C.c_int] + [C.c_double] * 3
     lib.lanes.argtypes, lib.lanes.restype = [C.c_ulonglong] * 2, C.c_uint
     return lib
 
@@ -53,3 +59,9 @@ def test_semi_infinite_with_two_blocks_per_sm(rules, mua, mus, pays, loses):
 def test_semi_infinite_at_the_crossing(rules):
     # 1.90 against 1.75 ms
     assert not rules.sub_lat(300_000, 1.0, 100.0, 2)
+
+
+@pytest.mark.parametrize("lo,hi,pays,loses", [(0.05, 2.0, 4_000, 20_000), (0.5, 5.0, 500, 3_000), (3.0, 30.0, 0, 2_000),
+                                              (0.05, 0.2, 3_000, 10_000)])
+def test_semi_infinite_sweep(rules, lo, hi, pays, loses):
+    assert (pays == 0 or rules.sweep_lat(351, pays, lo, hi)) and not rules.sweep_lat(351, loses, lo, hi)
