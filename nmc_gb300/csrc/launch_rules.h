@@ -54,10 +54,19 @@ inline bool sub_latency_pays(const WorkTail& w, int resident_blocks) {
   return w.below(resident_blocks >= kLatBlocks ? 1.2e5 : 3.7e4);
 }
 
-// The semi-infinite sweep's latency variant (two blocks are always resident).
-// 351 sets of mua in the range given, variant against the other: 0.05-2, 4e3
-// photons each 9.2 / 11.8 ms, 1e4 14.4 / 14.2; 0.5-5, 1e3 1.37 / 1.40, 3e3
-// 2.32 / 2.00, two-term 2e3 1.89 / 1.96, 4e3 3.20 / 2.53; 3-30, 1e3 0.43 / 0.38.
-inline bool sweep_latency_pays(const WorkTail& w) { return w.below(8e4); }
+// The semi-infinite sweep: finding a photon's set and loading its constants
+// costs about as much as 60 scatterings, which counts for short-lived sets.
+inline void sweep_add(WorkTail& w, double n, double mua, double mus) {
+  w.add(n, mua, mus);
+  w.work += 60.0 * n;
+}
+// Its latency variant (two blocks are always resident).  351 sets of mua in the
+// range given, variant against the other: 0.05-2, 4e3 photons each 9.2 / 11.8
+// ms, 1e4 14.4 / 14.2; 0.5-5, 1e3 1.37 / 1.40, 3e3 2.32 / 2.00, two-term 2e3
+// 1.89 / 1.96, 4e3 3.20 / 2.53; 3-30, 500 0.29 / 0.27, 1e3 0.43 / 0.38.  Spectra
+// with absorption bands, whose few long-lived sets are the tail, 3.5e6 photons
+// two-term: 24.2 / 31.8, 28.0 / 36.9 where the ratio is 1.0e5, 19.5 / 22.2 and
+// 19.6 / 18.3 at 1.25e5, 11.7 / 10.2 at 1.6e5.
+inline bool sweep_latency_pays(const WorkTail& w) { return w.below(1.1e5); }
 
 }  // namespace nmc

@@ -1271,7 +1271,7 @@ nmc_status nmc_run_sweep(nmc_handle* h, const nmc_sweep_set* sets, int32_t n_set
   const uint64_t warps = (uint64_t)h->nsm * nmc::kLatBlocks * (nmc::kLatBlock / 32);
   // the latency variant where it pays (launch_rules.h)
   nmc::WorkTail w;
-  for (int k = 0; k < n_sets; ++k) w.add((double)sets[k].photons, sets[k].mua, sets[k].mus);
+  for (int k = 0; k < n_sets; ++k) nmc::sweep_add(w, (double)sets[k].photons, sets[k].mua, sets[k].mus);
   const bool lat = h->ext.block_size <= 0 && h->ext.blocks_per_sm <= 0 && nmc::sweep_latency_pays(w);
   if (lat) p.lanes = nmc::lat_lanes(p.total, warps);
   const int block = h->ext.block_size > 0 ? h->ext.block_size : 256;

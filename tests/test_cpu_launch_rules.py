@@ -15,7 +15,12 @@ extern "C" {
 int sub_lat(double n, double mua, double mus, int blocks) { return sub_latency_pays(one(n, mua, mus), blocks); }
 int sweep_lat(int sets, double per, double lo, double hi) {
   WorkTail w;
-  for (int k = 0; k < sets; ++k) w.add(per, lo + (hi - lo) * k / (sets - 1), 100.0);
+  for (int k = 0; k < sets; ++k) sweep_add(w, per, lo + (hi - lo) * k / (sets - 1), 100.0);
+  return sweep_latency_pays(w);
+}
+int bands_lat(double clear, double per) {  // a share of the sets long-lived, the others not
+  WorkTail w;
+  for (int k = 0; k < 351; ++k) sweep_add(w, per, k < 351 * clear ? 0.05 : 2.0, 100.0);
   return sweep_latency_pays(w);
 }
 unsigned lanes(unsigned long long items, unsigned long long warps) { return lat_lanes(items, warps); }
@@ -32,6 +37,7 @@ def rules(tmp_path_factory):
     lib = C.CDLL(str(d / "rules.so"))
     lib.sub_lat.argtypes = [C.c_double] * 3 + [C.c_int]
     lib.sweep_lat.argtypes = [C.c_int] + [C.c_double] * 3
+    lib.bands_lat.argtypes = [C.c_double] * 2
     lib.lanes.argtypes, lib.lanes.restype = [C.c_ulonglong] * 2, C.c_uint
     return lib
 
@@ -65,3 +71,8 @@ def test_semi_infinite_at_the_crossing(rules):
                                               (0.05, 0.2, 3_000, 10_000)])
 def test_semi_infinite_sweep(rules, lo, hi, pays, loses):
     assert (pays == 0 or rules.sweep_lat(351, pays, lo, hi)) and not rules.sweep_lat(351, loses, lo, hi)
+
+
+def test_semi_infinite_sweep_of_bands(rules):
+    # the longest photons are a few sets': the work of the others is small beside that tail up to 1e4 photons each
+    assert rules.bands_lat(0.25, 8_000) and not rules.bands_lat(0.25, 30_000)
