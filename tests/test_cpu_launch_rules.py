@@ -4,6 +4,7 @@ import ctypes as C
 import os
 import subprocess
 
+import numpy as np
 import pytest
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
@@ -18,9 +19,9 @@ int sweep_lat(int sets, double per, double lo, double hi) {
   for (int k = 0; k < sets; ++k) sweep_add(w, per, lo + (hi - lo) * k / (sets - 1), 100.0);
   return sweep_latency_pays(w);
 }
-int bands_lat(double clear, double per) {  // a share of the sets long-lived, the others not
+int spectrum_lat(int n, const double* photons, const double* mua, const double* mus) {
   WorkTail w;
-  for (int k = 0; k < 351; ++k) sweep_add(w, per, k < 351 * clear ? 0.05 : 2.0, 100.0);
+  for (int k = 0; k < n; ++k) sweep_add(w, photons[k], mua[k], mus[k]);
   return sweep_latency_pays(w);
 }
 unsigned lanes(unsigned long long items, unsigned long long warps) { return lat_lanes(items, warps); }
@@ -37,7 +38,7 @@ def rules(tmp_path_factory):
     lib = C.CDLL(str(d / "rules.so"))
     lib.sub_lat.argtypes = [C.c_double] * 3 + [C.c_int]
     lib.sweep_lat.argtypes = [C.c_int] + [C.c_double] * 3
-    lib.bands_lat.argtypes = [C.c_double] * 2
+    lib.spectrum_lat.argtypes = [C.c_int] + [C.c_void_p] * 3
     lib.lanes.argtypes, lib.lanes.restype = [C.c_ulonglong] * 2, C.c_uint
     return lib
 
@@ -73,6 +74,15 @@ def test_semi_infinite_sweep(rules, lo, hi, pays, loses):
     assert (pays == 0 or rules.sweep_lat(351, pays, lo, hi)) and not rules.sweep_lat(351, loses, lo, hi)
 
 
-def test_semi_infinite_sweep_of_bands(rules):
-    # the longest photons are a few sets': the work of the others is small beside that tail up to 1e4 photons each
-    assert rules.bands_lat(0.25, 8_000) and not rules.bands_lat(0.25, 30_000)
+# spectra of 351 wavelengths, 3.51e6 photons, by seed: timed with the latency variant and without it (ms, two-term)
+@pytest.mark.parametrize("seed,variant,other", [(23, 26.3, 35.8), (16, 29.5, 39.3), (28, 17.6, 23.2), (3, 28.0, 36.9), (29, 23.5, 30.5),
+                                                (0, 24.2, 31.8), (26, 11.7, 10.2), (2, 11.3, 9.0), (18, 15.9, 13.4), (12, 14.1, 12.2),
+                                                (20, 14.7, 11.3), (27, 12.9, 9.9), (13, 8.6, 6.4), (17, 7.0, 5.1), (1, 9.5, 7.0)])
+def test_semi_infinite_sweep_of_spectra(rules, seed, variant, other):
+    from perf import cases
+
+    r = np.random.default_rng(seed)
+    w = np.exp(r.uniform(0.0, np.log(10.0), 351))
+    photons = np.maximum(1, (w / w.sum() * 3_510_000).astype(np.int64)).astype(np.float64)
+    mua, mus = (np.ascontiguousarray(q, np.float64) for q in cases._spectrum(r, 351, 0.05, 2.0, 0.05))
+    assert bool(rules.spectrum_lat(351, *(q.ctypes.data for q in (photons, mua, mus)))) == (variant < other)
