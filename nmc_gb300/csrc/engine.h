@@ -170,6 +170,7 @@ struct SweepParams {
   int phase_kind, fast;
   uint32_t step_cap;
   unsigned int lanes;  // > 0: the latency variant, with this many lanes of a warp taking photons
+  int full;            // one-term, not the latency variant: four blocks per SM
 };
 
 cudaError_t launch_sweep(const SweepParams& p, int grid, int block, cudaStream_t stream);

@@ -68,5 +68,11 @@ inline void sweep_add(WorkTail& w, double n, double mua, double mus) {
 // two-term: 24.2 / 31.8, 28.0 / 36.9 where the ratio is 1.0e5, 19.5 / 22.2 and
 // 19.6 / 18.3 at 1.25e5, 11.7 / 10.2 at 1.6e5.
 inline bool sweep_latency_pays(const WorkTail& w) { return w.below(1.1e5); }
+// Without it, the one-term sweep runs 4 blocks of 64 registers per SM from this
+// ratio on, 3 of 74-78 below (two-term keeps 3: it spills at 4).  3 blocks
+// against 4: mua 3-30, 3e4 photons each 7.90 / 7.27 ms; 0.5-5, 1e4 5.55 / 5.47,
+// 3e4 16.5 / 15.7; 0.05-2, 3e4 26.6 / 28.9, 1e5 88.2 / 85.3; 0.05-0.2, 1e4
+// 24.4 / 28.9, 3e4 63.8 / 66.8, 1e5 208 / 205: they cross at 5e5 to 1e6.
+inline bool sweep_fills_sm(const WorkTail& w) { return !w.below(7e5); }
 
 }  // namespace nmc

@@ -1274,6 +1274,7 @@ nmc_status nmc_run_sweep(nmc_handle* h, const nmc_sweep_set* sets, int32_t n_set
   for (int k = 0; k < n_sets; ++k) nmc::sweep_add(w, (double)sets[k].photons, sets[k].mua, sets[k].mus);
   const bool lat = h->ext.block_size <= 0 && h->ext.blocks_per_sm <= 0 && nmc::sweep_latency_pays(w);
   if (lat) p.lanes = nmc::lat_lanes(p.total, warps);
+  p.full = nmc::sweep_fills_sm(w) ? 1 : 0;
   const int block = h->ext.block_size > 0 ? h->ext.block_size : 256;
   int per_sm = 0;
   if (nmc::sweep_occupancy(p, block, &per_sm) != cudaSuccess || per_sm < 1)

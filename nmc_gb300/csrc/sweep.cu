@@ -32,9 +32,9 @@
 namespace nmc {
 namespace {
 
-// LAT: the latency variant (engine.h).
-template <int PHASE, bool FAST, bool LAT>
-__global__ void __launch_bounds__(kLatBlock, LAT ? kLatBlocks : 3) sweep_kernel(const SweepParams P) {
+// LAT: the latency variant; FULL: four blocks per SM (launch_rules.h).
+template <int PHASE, bool FAST, bool LAT, bool FULL = false>
+__global__ void __launch_bounds__(kLatBlock, LAT ? kLatBlocks : FULL ? 4 : 3) sweep_kernel(const SweepParams P) {
   using M = Math<FAST>;
   constexpr bool TT = PHASE == kPhaseTT;
   extern __shared__ unsigned long long s_sum[];  // nsets x 5: photons, hops, S, A, E
@@ -277,7 +277,9 @@ __global__ void __launch_bounds__(kLatBlock, LAT ? kLatBlocks : 3) sweep_kernel(
 }
 
 template <bool FAST, bool LAT>
-const void* pick(int phase) {
+const void* pick(int phase, bool full) {
+  if (!LAT && full && phase == kPhaseHG) return (const void*)sweep_kernel<kPhaseHG, FAST, false, true>;
+  if (!LAT && full && phase == kPhaseIsoRef) return (const void*)sweep_kernel<kPhaseIsoRef, FAST, false, true>;
   if (phase == kPhaseTT) return (const void*)sweep_kernel<kPhaseTT, FAST, LAT>;
   if (phase == kPhaseIsoRef) return (const void*)sweep_kernel<kPhaseIsoRef, FAST, LAT>;
   return (const void*)sweep_kernel<kPhaseHG, FAST, LAT>;
@@ -289,9 +291,9 @@ size_t sweep_smem_bytes(int nsets) { return (size_t)nsets * 6 * 8; }
 
 cudaError_t sweep_prepare(const SweepParams& p, const void** f, size_t* sh) {
   if (p.lanes > 0)
-    *f = p.fast ? pick<true, true>(p.phase_kind) : pick<false, true>(p.phase_kind);
+    *f = p.fast ? pick<true, true>(p.phase_kind, false) : pick<false, true>(p.phase_kind, false);
   else
-    *f = p.fast ? pick<true, false>(p.phase_kind) : pick<false, false>(p.phase_kind);
+    *f = p.fast ? pick<true, false>(p.phase_kind, p.full) : pick<false, false>(p.phase_kind, p.full);
   *sh = sweep_smem_bytes(p.nsets);
   // a block's static shared memory counts against the 48 KB it has without
   // this; 1024 sets alone take all of it

@@ -19,6 +19,11 @@ int sweep_lat(int sets, double per, double lo, double hi) {
   for (int k = 0; k < sets; ++k) sweep_add(w, per, lo + (hi - lo) * k / (sets - 1), 100.0);
   return sweep_latency_pays(w);
 }
+int sweep_full(int sets, double per, double lo, double hi) {
+  WorkTail w;
+  for (int k = 0; k < sets; ++k) sweep_add(w, per, lo + (hi - lo) * k / (sets - 1), 100.0);
+  return sweep_fills_sm(w);
+}
 int spectrum_lat(int n, const double* photons, const double* mua, const double* mus) {
   WorkTail w;
   for (int k = 0; k < n; ++k) sweep_add(w, photons[k], mua[k], mus[k]);
@@ -37,7 +42,7 @@ def rules(tmp_path_factory):
                     "-o", str(d / "rules.so")], check=True)
     lib = C.CDLL(str(d / "rules.so"))
     lib.sub_lat.argtypes = [C.c_double] * 3 + [C.c_int]
-    lib.sweep_lat.argtypes = [C.c_int] + [C.c_double] * 3
+    lib.sweep_full.argtypes = lib.sweep_lat.argtypes = [C.c_int] + [C.c_double] * 3
     lib.spectrum_lat.argtypes = [C.c_int] + [C.c_void_p] * 3
     lib.lanes.argtypes, lib.lanes.restype = [C.c_ulonglong] * 2, C.c_uint
     return lib
@@ -86,3 +91,9 @@ def test_semi_infinite_sweep_of_spectra(rules, seed, variant, other):
     photons = np.maximum(1, (w / w.sum() * 3_510_000).astype(np.int64)).astype(np.float64)
     mua, mus = (np.ascontiguousarray(q, np.float64) for q in cases._spectrum(r, 351, 0.05, 2.0, 0.05))
     assert bool(rules.spectrum_lat(351, *(q.ctypes.data for q in (photons, mua, mus)))) == (variant < other)
+
+
+@pytest.mark.parametrize("lo,hi,three,four", [(3.0, 30.0, 1_000, 10_000), (0.5, 5.0, 3_000, 30_000), (0.05, 2.0, 10_000, 100_000),
+                                              (0.05, 0.2, 10_000, 100_000)])
+def test_one_term_sweep_fills_the_sm(rules, lo, hi, three, four):
+    assert not rules.sweep_full(351, three, lo, hi) and rules.sweep_full(351, four, lo, hi)

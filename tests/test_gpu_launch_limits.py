@@ -59,3 +59,23 @@ def test_semi_infinite_with_one_block_per_sm(gpu, rng, n):
         assert got[0][0][k] == got[1][0][k], k
     for k in got[0][1]:
         np.testing.assert_array_equal(got[0][1][k], got[1][1][k], err_msg=k)
+
+
+@pytest.mark.parametrize("phase", [abi.PHASE_HG, abi.PHASE_ISOTROPIC_REF])
+def test_sweep_that_fills_the_gpu_gives_the_parts(gpu, phase):
+    # 8 short-lived sets of 120,000 photons take four blocks per SM, a 24th of them the latency variant
+    # and a sixth the kernel of three blocks: the same photons, the same integer sums
+    def sets(n, first):
+        return [abi.SweepSet(mua=10.0 + k, mus=60.0 + k, g=0.8, gf=0.9, af=0.5, gb=0.3, ab=0.5, cc=0.9, n1=1.37, n2=1.0, pad=0, photons=n,
+                             first_photon=first) for k in range(8)]
+    rp, tp, ext = cases.mcsub_case(phase=phase, seed=5)
+    n = 120_000
+    with gpu.Engine(abi.SIM_MCSUB, 0, ext) as e:
+        e.prepare_data(rp, tp)
+        whole = e.run_sweep(sets(n, 3), with_J=True)
+        for parts in (6, 24):
+            got = [e.run_sweep(sets(n // parts, 3 + k * (n // parts)), with_J=True) for k in range(parts)]
+            for q in ("photons", "hops", "J"):
+                np.testing.assert_array_equal(whole[q], sum(g[q] for g in got), err_msg=q)
+            for q in ("S", "A", "E", "E2"):
+                np.testing.assert_allclose(whole[q], sum(g[q] for g in got), rtol=1e-12, err_msg=q)
