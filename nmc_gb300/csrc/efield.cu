@@ -1031,11 +1031,11 @@ extern "C" nmc_status nmc_efield_run(int32_t device, const nmc_efield_config* cf
   const bool fast = !(c.flags & NMC_FLAG_PRECISE_MATH);
   int nsm = 0;
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device);
-  const unsigned long long warps = (unsigned long long)nsm * kLatBlocks * (kLatBlock / 32);
-  // Up to 32 photons per lane of the latency variant it is the faster one (8
-  // settings, about 5,300 scatterings per photon and up to 95,000: 800 photons
-  // take 59 against 88 ms, 8e4 127 / 169, 1e6 205 / 291, 2e6 307 / 342, 4e6
-  // 531 / 513 ms).
+  // The latency variant where it pays (launch_rules.h); the photons that are
+  // converted live on in the second medium.
+  WorkTail w;
+  w.add((double)P.total, (double)c.mua + c.mu_raman, c.mus);
+  if (raman) w.add((double)P.total * c.mu_raman / ((double)c.mua + c.mu_raman), c.raman_mua, c.raman_mus);
   // The tables (8 bytes per angle) share a block's memory with the kernel's
   // static arrays; the latency variant has 32 bytes more of them, so the last
   // sizes that fit a block at all (27,003 to 27,006 angles) take the other one.
@@ -1050,8 +1050,7 @@ extern "C" nmc_status nmc_efield_run(int32_t device, const nmc_efield_config* cf
     cudaFuncAttributes a{};
     return cudaFuncGetAttributes(&a, k) == cudaSuccess && a.sharedSizeBytes + smem <= (size_t)max_smem;
   };
-  const bool lat = P.total <= warps * 32 * 32 && fits(kernel(true));
-  P.lanes = (unsigned int)std::max<unsigned long long>(1, std::min<unsigned long long>(32, (P.total + warps - 1) / warps));
+  const bool lat = field_latency_pays(w, P.total, (uint64_t)nsm * kLatBlocks * (kLatBlock / 32)) && fits(kernel(true));
   const void* f = kernel(lat);
   // above 48 KB together with the static arrays a block must ask for it
   if (smem > 16 * 1024 && cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
@@ -1061,6 +1060,7 @@ extern "C" nmc_status nmc_efield_run(int32_t device, const nmc_efield_config* cf
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f, 256, smem) != cudaSuccess || per_sm < 1)
     return done(NMC_EDEVICE);
   if (lat) per_sm = std::min(per_sm, kLatBlocks);
+  P.lanes = lat_lanes(P.total, (uint64_t)nsm * per_sm * (kLatBlock / 32));  // of the warps that are resident
   const unsigned long long grid = std::max<unsigned long long>(
       1, std::min<unsigned long long>((unsigned long long)nsm * per_sm, lat ? P.total : (P.total + 255) / 256));
   void* args[] = {(void*)&P};

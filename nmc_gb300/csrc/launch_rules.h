@@ -75,4 +75,13 @@ inline bool sweep_latency_pays(const WorkTail& w) { return w.below(1.1e5); }
 // 24.4 / 28.9, 3e4 63.8 / 66.8, 1e5 208 / 205: they cross at 5e5 to 1e6.
 inline bool sweep_fills_sm(const WorkTail& w) { return !w.below(7e5); }
 
+// The E-field kernel's latency variant, up to 32 photons per lane.  8 settings,
+// variant against the other, photons each: mua 0.01, 1e5 191 / 289 ms, 3.1e5 345
+// / 381, 6e5 575 / 563; mua 0.1, 1e5 34.6 / 37.2, 2e5 60.4 / 56.7; mua 1, 2e4
+// 2.6 / 3.4, 5e4 4.9 / 4.8, 1e5 8.2 / 7.4; mua 10, 1e4 0.59 / 0.61, 5e4 1.26 /
+// 1.15, 3.1e5 5.8 / 4.2: they cross at 1.1e5 to 2.5e5.
+inline bool field_latency_pays(const WorkTail& w, uint64_t photons, uint64_t warps) {
+  return photons <= warps * 32 * 32 && w.below(1.6e5);
+}
+
 }  // namespace nmc

@@ -29,6 +29,7 @@ int spectrum_lat(int n, const double* photons, const double* mua, const double* 
   for (int k = 0; k < n; ++k) sweep_add(w, photons[k], mua[k], mus[k]);
   return sweep_latency_pays(w);
 }
+int field_lat(double n, double mua) { return field_latency_pays(one(n, mua, 100.0), (uint64_t)n, 2432); }
 unsigned lanes(unsigned long long items, unsigned long long warps) { return lat_lanes(items, warps); }
 }
 """
@@ -44,6 +45,7 @@ def rules(tmp_path_factory):
     lib.sub_lat.argtypes = [C.c_double] * 3 + [C.c_int]
     lib.sweep_full.argtypes = lib.sweep_lat.argtypes = [C.c_int] + [C.c_double] * 3
     lib.spectrum_lat.argtypes = [C.c_int] + [C.c_void_p] * 3
+    lib.field_lat.argtypes = [C.c_double] * 2
     lib.lanes.argtypes, lib.lanes.restype = [C.c_ulonglong] * 2, C.c_uint
     return lib
 
@@ -97,3 +99,9 @@ def test_semi_infinite_sweep_of_spectra(rules, seed, variant, other):
                                               (0.05, 0.2, 10_000, 100_000)])
 def test_one_term_sweep_fills_the_sm(rules, lo, hi, three, four):
     assert not rules.sweep_full(351, three, lo, hi) and rules.sweep_full(351, four, lo, hi)
+
+
+@pytest.mark.parametrize("mua,pays,loses", [(0.01, 8 * 100_000, 8 * 2_000_000), (0.1, 8 * 50_000, 8 * 310_000), (1.0, 8 * 20_000, 8 * 100_000),
+                                            (10.0, 8 * 5_000, 8 * 100_000), (100.0, 8 * 2_000, 8 * 100_000)])
+def test_field(rules, mua, pays, loses):
+    assert rules.field_lat(pays, mua) and not rules.field_lat(loses, mua)
