@@ -84,4 +84,49 @@ inline bool field_latency_pays(const WorkTail& w, uint64_t photons, uint64_t war
   return photons <= warps * 32 * 32 && w.below(1.6e5);
 }
 
+// A plane layer as the rule sees it.
+struct PlaneLayer {
+  double mua, mus, g, thickness;
+};
+
+// n photons in a stack: the longest live in the layer with the most scatterings
+// per absorption, where leaving the layer counts as absorption at the rate of
+// its slowest diffusion mode, D (pi / L)^2, L the thickness and 6 D beyond each
+// face (a refractive step of 1.4).  Layers below nine effective attenuation
+// lengths are out of reach, layers that do not scatter hold no walk.
+inline void layered_add(WorkTail& w, double n, const PlaneLayer* layers, int n_layers) {
+  double best = 1.0, depth = 0.0;
+  for (int l = 0; l < n_layers && depth < 9.2; ++l) {
+    const PlaneLayer& q = layers[l];
+    const double tr = q.mua + q.mus * (1.0 - q.g);  // transport coefficient
+    if (q.mus > 0.0 && tr > 0.0) {
+      const double D = 1.0 / (3.0 * tr);
+      double loss = q.mua;
+      if (std::isfinite(q.thickness)) loss += D * std::pow(3.14159265358979 / (q.thickness + 12.0 * D), 2);
+      best = std::max(best, (loss + q.mus) / std::max(loss, 1e-6));
+    }
+    depth += std::sqrt(3.0 * q.mua * tr) * q.thickness;
+  }
+  w.add(n, 1.0, best - 1.0);
+}
+
+// The layered kernel's variant and blocks per SM (0: as many as fit, four).
+// * Up to kThinPhotons per warp, where every photon has helper lanes from the
+//   start, the latency variant: three-layer skin 1e3 photons 5.1 against 5.8 ms,
+//   1e4 7.1 / 7.4, 2e4 7.5 / 7.7, 4e4 8.3 / 7.7; mua 10-20 1e4 0.34 / 0.38.
+// * Up to eight photons per lane, while the tail outweighs the work, two blocks
+//   of the other one.  2 against 4 blocks: skin 3e5 11.0 / 14.2 ms, 6e5 14.9 /
+//   15.6, 1e6 21.4 / 19.7; mua 1, mus 100 2e5 1.68 / 1.78, 3e5 2.20 / 2.02; mua
+//   10-20 6e4 0.41 / 0.40, 1e5 0.45 / 0.43, 6e5 1.09 / 0.84; 0.3 cm without
+//   absorption 2e5 1.12 / 1.14, 3e5 1.40 / 1.31; gradients and the reference's
+//   streams cross at the same sizes: at 0.7e5 to 1.2e5.
+struct LayeredShape {
+  bool latency;
+  int blocks;
+};
+inline LayeredShape layered_shape(const WorkTail& w, uint64_t photons, uint64_t warps, bool sequential) {
+  if (!sequential && photons <= warps * kThinPhotons) return {true, kLatBlocks};
+  return {false, photons <= warps * 256 && w.below(1.0e5) ? kLatBlocks : 0};
+}
+
 }  // namespace nmc

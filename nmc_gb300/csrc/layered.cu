@@ -514,11 +514,15 @@ nmc_status layered_impl(int32_t device, const nmc_layered_config* cfg, const nmc
   int nsm = 0;
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device);
   const unsigned long long warps = (unsigned long long)nsm * kLatBlocks * (kLatBlock / 32);
-  // Up to four photons per lane of the latency variant it is the faster one
-  // (three-layer skin: 1e3 photons 6.0 against 6.7 ms, 1e5 9.6 / 10.1, 3e5 14.1
-  // / 15.5, 1e6 24.7 / 20.8 ms); the reference's generator is sequential.
-  const bool lat = !ref && photons <= warps * 128;
-  P.lanes = (unsigned int)std::max<unsigned long long>(1, std::min<unsigned long long>(32, (photons + warps - 1) / warps));
+  // variant and blocks per SM by launch_rules.h; the reference's generator is sequential
+  std::vector<PlaneLayer> plane;
+  for (int l = 0; l < c.n_layers; ++l)
+    plane.push_back({layers[l].mua, layers[l].mus, iso ? 0.0 : (double)layers[l].g, layers[l].thickness});
+  WorkTail w;
+  layered_add(w, (double)photons, plane.data(), c.n_layers);
+  const LayeredShape shape = layered_shape(w, photons, warps, ref);
+  const bool lat = shape.latency;
+  P.lanes = lat_lanes(photons, warps);
 #define NMC_LAYERED(ADJ, REF, LAT) \
   (fast ? (const void*)layered_kernel<true, ADJ, REF, LAT> : (const void*)layered_kernel<false, ADJ, REF, LAT>)
   const void* f = adj   ? (lat ? NMC_LAYERED(true, false, true) : NMC_LAYERED(true, false, false))
@@ -534,12 +538,7 @@ nmc_status layered_impl(int32_t device, const nmc_layered_config* cfg, const nmc
   int per_sm = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f, 256, smem) != cudaSuccess || per_sm < 1)
     return done(NMC_EDEVICE);
-  // Up to eight photons per lane of two blocks per SM, the throughput variant
-  // also runs two: the tail of long photons is most of the run, and among
-  // fewer warps a step takes less time (three-layer skin at 2 / 4 blocks: 3.2e5
-  // photons 13.6 / 16 ms, 5e5 14.8 / 16.3, 6e5 15.8 / 17.1; adjoint 6e5 20.0 /
-  // 21.4; reference streams 1e5 8.8 / 10.5; 1e6 21.2 / 20.3).
-  if (photons <= warps * 256) per_sm = std::min(per_sm, kLatBlocks);
+  if (shape.blocks > 0) per_sm = std::min(per_sm, shape.blocks);
   const unsigned long long grid = std::max<unsigned long long>(
       1, std::min<unsigned long long>((unsigned long long)nsm * per_sm, lat ? photons : (photons + 255) / 256));
   void* args[] = {(void*)&P};

@@ -30,6 +30,12 @@ int spectrum_lat(int n, const double* photons, const double* mua, const double* 
   return sweep_latency_pays(w);
 }
 int field_lat(double n, double mua) { return field_latency_pays(one(n, mua, 100.0), (uint64_t)n, 2432); }
+int layered(unsigned long long n, int nl, const double* q, int ref) {  // 0: the latency variant, else blocks per SM
+  WorkTail w;
+  layered_add(w, (double)n, reinterpret_cast<const PlaneLayer*>(q), nl);
+  const LayeredShape s = layered_shape(w, n, 2432, ref);
+  return s.latency ? 0 : s.blocks ? s.blocks : 4;
+}
 unsigned lanes(unsigned long long items, unsigned long long warps) { return lat_lanes(items, warps); }
 }
 """
@@ -46,6 +52,7 @@ def rules(tmp_path_factory):
     lib.sweep_full.argtypes = lib.sweep_lat.argtypes = [C.c_int] + [C.c_double] * 3
     lib.spectrum_lat.argtypes = [C.c_int] + [C.c_void_p] * 3
     lib.field_lat.argtypes = [C.c_double] * 2
+    lib.layered.argtypes = [C.c_ulonglong, C.c_int, C.c_void_p, C.c_int]
     lib.lanes.argtypes, lib.lanes.restype = [C.c_ulonglong] * 2, C.c_uint
     return lib
 
@@ -105,3 +112,30 @@ def test_one_term_sweep_fills_the_sm(rules, lo, hi, three, four):
                                             (10.0, 8 * 5_000, 8 * 100_000), (100.0, 8 * 2_000, 8 * 100_000)])
 def test_field(rules, mua, pays, loses):
     assert rules.field_lat(pays, mua) and not rules.field_lat(loses, mua)
+
+
+INF = float("inf")
+STACKS = {  # (mua, mus, g, thickness), the last size at which two blocks were not slower, the first at which four were faster by 5%
+    "skin": ([(3.0, 200.0, 0.8, 0.01), (0.3, 150.0, 0.85, 0.2), (0.1, 100.0, 0.9, INF)], 600_000, 1_000_000),
+    "epidermis": ([(3.0, 200.0, 0.8, INF)], 100_000, 300_000),
+    "mua_1": ([(1.0, 100.0, 0.9, INF)], 200_000, 450_000),
+    "absorbing": ([(10.0, 100.0, 0.9, 0.05), (20.0, 100.0, 0.9, INF)], 60_000, 200_000),
+    "no_absorption": ([(0.0, 100.0, 0.9, 0.3)], 200_000, 300_000),
+    "no_absorption_thick": ([(0.0, 100.0, 0.9, 2.0)], 600_000, INF),
+    "no_absorption_over": ([(0.0, 100.0, 0.9, 0.3), (1.0, 100.0, 0.9, INF)], 200_000, 450_000),
+    "clear_gap": ([(1.0, 80.0, 0.9, 0.03), (0.0, 0.0, 0.0, 0.02), (1.0, 80.0, 0.9, 0.05)], 60_000, 200_000),
+    "out_of_reach": ([(20.0, 100.0, 0.8, 0.5), (0.05, 100.0, 0.9, INF)], 60_000, 200_000),
+}
+
+
+@pytest.mark.parametrize("name", STACKS)
+def test_layered(rules, name):
+    q, two, four = STACKS[name]
+    a = np.array(q, np.float64)
+    for ref in (0, 1):
+        assert rules.layered(two, len(q), a.ctypes.data, ref) == 2
+        assert four == INF or rules.layered(four, len(q), a.ctypes.data, ref) == 4
+    for n in (1, 1000, 19_456):
+        assert rules.layered(n, len(q), a.ctypes.data, 0) == 0
+        assert rules.layered(n, len(q), a.ctypes.data, 1) != 0
+    assert rules.layered(40_000, len(q), a.ctypes.data, 0) != 0

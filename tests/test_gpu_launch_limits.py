@@ -79,3 +79,18 @@ def test_sweep_that_fills_the_gpu_gives_the_parts(gpu, phase):
                 np.testing.assert_array_equal(whole[q], sum(g[q] for g in got), err_msg=q)
             for q in ("S", "A", "E", "E2"):
                 np.testing.assert_allclose(whole[q], sum(g[q] for g in got), rtol=1e-12, err_msg=q)
+
+
+@pytest.mark.parametrize("adjoint", [False, True])
+def test_layered_variants_follow_the_same_photons(gpu, adjoint):
+    # 8 photons per warp are the latency variant's last size, three times as many the other kernel's
+    from nmc_gb300 import layered
+
+    stack, n = [(3.0, 200.0, 0.8, 1.4, 0.01), (0.0, 0.0, 0.0, 1.5, 0.02), (0.3, 150.0, 0.85, 1.4, 0.2), (0.1, 100.0, 0.9, 1.44, float("inf"))], 19_456
+    up = np.linspace(-1.0, 1.0, 51).astype(np.float32)
+    run = (lambda m, f: layered.adjoint(stack, m, grad_rd_r=up, nr=50, dr=0.02, seed=3, first=f)) if adjoint else \
+          (lambda m, f: layered.run(stack, m, nr=50, dr=0.02, nz=70, dz=0.01, seed=3, first=f, a_rz=True))
+    whole, parts = run(3 * n, 11), [run(n, 11 + k * n) for k in range(3)]
+    for k in ("photons", "Rd", "Rd2", "Tt", "A", "interactions", "rd_r", "tt_r") + (
+            ("grad_mua", "grad_mus", "grad_g") if adjoint else ("a_z", "a_rz", "a_layer")):
+        np.testing.assert_allclose(whole[k], sum(p[k] for p in parts), rtol=1e-11, atol=1e-9, err_msg=k)
