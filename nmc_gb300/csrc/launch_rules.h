@@ -6,6 +6,8 @@
 #include <cmath>
 #include <cstdint>
 
+#include "nmc_abi.h"
+
 namespace nmc {
 
 // The latency variant of a kernel runs few photons per lane: kLatBlocks blocks
@@ -127,6 +129,56 @@ struct LayeredShape {
 inline LayeredShape layered_shape(const WorkTail& w, uint64_t photons, uint64_t warps, bool sequential) {
   if (!sequential && photons <= warps * kThinPhotons) return {true, kLatBlocks};
   return {false, photons <= warps * 256 && w.below(1.0e5) ? kLatBlocks : 0};
+}
+
+// n photons in a voxel grid whose longest side is `extent` and whose map holds
+// the tissues of `present` (bit t: tissue t): the longest live in the tissue with
+// the most scatterings per absorption.  A tissue too clear to turn a photon within
+// the grid (air) holds no walk.
+inline void voxel_add(WorkTail& w, double n, const nmc_tissue_params& tp, bool two_term, uint32_t present, double extent) {
+  double best = 1.0;
+  for (int t = 0; t < NMC_NTISS; ++t) {
+    if (!(present >> t & 1u)) continue;
+    const double g = two_term ? tp.CC[t] * tp.gf[t] - (1.0 - tp.CC[t]) * tp.gb[t] : (double)tp.gv[t];
+    const double mua = tp.muav[t], mus = tp.musv[t];
+    if (mus * (1.0 - g) * extent >= 1.0) best = std::max(best, (mua + mus) / std::max(mua, 1e-6));
+  }
+  w.add(n, 1.0, best - 1.0);
+}
+
+// The launch shape of a voxel run whose caller left it to the library, from
+// its queue items (photons, or runs of photons) and work against tail.  A voxel
+// sub-step takes a lone photon 0.49 us, a photon in a full warp 1.4 us (its 31
+// neighbours walk other branches) and one of eight full warps on a scheduler 2
+// us, and 4, 6, 8 warps per scheduler give 77, 94, 100% of the throughput:
+//  * up to 5 items per warp of two blocks per SM, each warp takes as few items
+//    as fill them all (blocks of that many threads): 1e3 photons through the
+//    skin-vessel map take 5.9 instead of 10.1 ms, 1e4 8.7 / 10.2;
+//  * 2 or 3 blocks per SM while the tail outweighs the work and photons per lane
+//    are few (where the estimate from the table may miss a tissue that few photons
+//    reach).  2 / 3 / 4 blocks: skin vessel 1e5 13.9 / 15.7 / 15.5 ms, 2e5 16.8 /
+//    17.4 / 20.8, 3e5 21.4 / 20.4 / 23.3, 1e6 48.2 / 42.9 / 43.5; a cube of mua 1
+//    1e5 3.00 / 3.17 / 3.10, 2e5 4.66 / 4.46 / 4.63; mua 20 1e5 0.26 / 0.21 /
+//    0.21, 4e5 0.80 / 0.65 / 0.61; mua 50 2e5 0.19 / 0.15 / 0.14;
+//  * a sweep's sets differ and its tail is longer.  351 sets of the skin vessel,
+//    one-term 1.4e6 69 / 77 / 94, 2.5e6 120 / 99 / 113, 5e6 239 / 193 / 186; two-
+//    term 1.4e6 57 / 66 / 80, 3.5e6 70 / 78 / 96, 7e6 136 / 110 / 120, other
+//    spectra at 3.5e6 64 / 57 / 62 and 92 / 100 / 120; with 20 times the
+//    absorption one-term 1.4e6 7.6 / 7.0 / 7.2, 3.5e6 17.3 / 14.0 / 13.5;
+//  * photons that end at the grid's faces (boundaryflag 1) run on all blocks that
+//    fit: how long they live is the grid's size rather than the table's.  Grids
+//    that hold them do have the tail (a 2 cm cube of mua 1, 1e5 photons 2.50 /
+//    2.66 / 2.68 ms, 3e5 5.14 / 4.72 / 4.83), small ones do not.
+struct VoxelShape {
+  int block, per_sm;
+};
+inline VoxelShape voxel_shape(const WorkTail& w, uint64_t items, int nsm, bool ends_at_faces, bool sweep) {
+  const uint64_t warps = (uint64_t)nsm * kLatBlocks * (kLatBlock / 32), lanes = warps * 32;
+  if (items <= 5 * warps) return {(int)std::max<uint64_t>(1, (items + warps - 1) / warps), 16};
+  if (ends_at_faces) return {256, 4};
+  if ((sweep ? items <= 26 * lanes : 2 * items <= 3 * lanes) && w.below(sweep ? 1.0e5 : 5e4)) return {256, 2};
+  if (items <= (sweep ? 64 : 5) * lanes && w.below(2.7e5)) return {256, 3};
+  return {256, 4};
 }
 
 }  // namespace nmc

@@ -95,6 +95,7 @@ struct nmc_handle {
   // per-voxel media, radial tally, adjoint
   bool voxel_mode = false;
   float4* d_vox = nullptr;
+  double vox_mua = 0.0, vox_mus = 0.0;  // their means
   int rd_bins = 0;
   float rd_dr = 0.f;
   unsigned long long* d_rdr = nullptr;
@@ -394,29 +395,9 @@ struct AdjArgs {
 
 nmc_status fold(nmc_handle* h);
 
-// The launch shape of a voxel run whose caller left it to the library, from
-// its queue items (photons, or runs of photons).  A voxel sub-step takes a lone
-// photon 0.49 us, a photon in a full warp 1.4 us (its 31 neighbours walk other
-// branches) and one of eight full warps on a scheduler 2 us, so:
-//  * up to 5 items per warp of two blocks per SM, each warp takes as few items
-//    as fill them all (blocks of that many threads): 1e3 photons through the
-//    skin-vessel map take 5.9 instead of 10.1 ms, 1e4 8.7 / 10.2;
-//  * while photons per lane are few the tail of long photons outweighs the
-//    throughput that more warps give (4, 6, 8 warps per scheduler: 77, 94,
-//    100%): 1e5 photons take 14.7 / 16.8 / 16.4 ms at 2, 3, 4 blocks per SM,
-//    3e5 20.3 / 20.5 / 23.1, 1e6 48 / 42 / 43; a sweep's sets differ and its
-//    tail is longer: 1.4e6 photons 45-67 / 54-80 / 67-98 ms, 3.5e6 60-82 /
-//    62-93 / 76-113, 7e6 119-144 / 96-123 / 92-136;
-//  * photons that end at the grid's faces (boundaryflag 1) have no such tail.
-struct VoxelShape {
-  int block, per_sm;
-};
-VoxelShape voxel_shape(const nmc_handle* h, uint64_t items, bool sweep) {
-  const uint64_t warps = (uint64_t)h->nsm * 2 * (256 / 32), lanes = warps * 32;
-  if (items <= 5 * warps) return {(int)std::max<uint64_t>(1, (items + warps - 1) / warps), 16};
-  if (h->rp.boundaryflag == 1) return {256, 4};
-  if (sweep) return {256, items <= 26 * lanes ? 2 : items <= 64 * lanes ? 3 : 4};
-  return {256, 2 * items <= 3 * lanes ? 2 : items <= 5 * lanes ? 3 : 4};
+// The longest side of the handle's grid.
+double grid_extent(const nmc_run_params& rp) {
+  return std::max({(double)rp.Nx * rp.dx, (double)rp.Ny * rp.dy, (double)rp.Nz * rp.dz});
 }
 
 nmc_status launch(nmc_handle* h, uint64_t first, uint64_t n, nmc_photon_record* d_recs,
@@ -498,9 +479,15 @@ nmc_status launch(nmc_handle* h, uint64_t first, uint64_t n, nmc_photon_record* 
       }
     }
     const bool own = !trace && h->ext.block_size <= 0 && h->ext.blocks_per_sm <= 0;
-    const VoxelShape shape = voxel_shape(h, (n + p.per_fetch - 1) / p.per_fetch, false);
-    block = own ? shape.block : h->ext.block_size > 0 ? h->ext.block_size : 256;
     const bool tt = h->sim == NMC_SIM_MCXYZ_TT;
+    nmc::WorkTail w;
+    if (h->voxel_mode)
+      w.add((double)n, h->vox_mua, h->vox_mus);
+    else
+      nmc::voxel_add(w, (double)n, h->tp, tt, h->tiss_used, grid_extent(h->rp));
+    const nmc::VoxelShape shape =
+        nmc::voxel_shape(w, (n + p.per_fetch - 1) / p.per_fetch, h->nsm, h->rp.boundaryflag == 1, false);
+    block = own ? shape.block : h->ext.block_size > 0 ? h->ext.block_size : 256;
     const int mode = !adj ? nmc::kVoxel : adj->pass == 0 ? nmc::kRecord : adj->pass == 2 ? nmc::kScore : nmc::kAdjoint;
     if (h->voxel_mode)
       NMC_CUDA(h, nmc::mcxyz_voxel_occupancy(mode, trace, block, &per_sm));
@@ -1405,7 +1392,11 @@ nmc_status nmc_run_sweep_tissues(nmc_handle* h, const nmc_tissue_params* tables,
     return fail(h, NMC_EDEVICE, "sweep buffer set-up");
   const bool tt = h->sim == NMC_SIM_MCXYZ_TT;
   const bool own = h->ext.block_size <= 0 && h->ext.blocks_per_sm <= 0;
-  const VoxelShape shape = voxel_shape(h, (p.n + p.per_fetch - 1) / p.per_fetch, true);
+  nmc::WorkTail w;
+  for (int s = 0; s < n_sets; ++s)
+    nmc::voxel_add(w, (double)photons[s], tables[s], tt, h->tiss_used, grid_extent(h->rp));
+  const nmc::VoxelShape shape =
+      nmc::voxel_shape(w, (p.n + p.per_fetch - 1) / p.per_fetch, h->nsm, h->rp.boundaryflag == 1, true);
   const int block = own ? shape.block : h->ext.block_size > 0 ? h->ext.block_size : 256;
   int per_sm = 0;
   if (nmc::mcxyz_sweep_occupancy(tt, block, &per_sm) != cudaSuccess || per_sm < 1)
@@ -1452,6 +1443,7 @@ nmc_status nmc_set_voxel_props(nmc_handle* h, const float* mua, const float* mus
   if (st != NMC_OK && st != NMC_ESTEPCAP) return st;
   std::vector<float4> v(h->nvox);
   const float g1 = h->tp.gv[1];
+  double sum_a = 0.0, sum_s = 0.0;
   for (size_t k = 0; k < h->nvox; ++k) {
     const float a = mua[k], s = mus[k], gg = g ? g[k] : g1;
     if (!std::isfinite(a) || a < 0.f || !std::isfinite(s) || !(s > 0.f) || !std::isfinite(gg) || !(gg > -1.f) ||
@@ -1461,9 +1453,13 @@ nmc_status nmc_set_voxel_props(nmc_handle* h, const float* mua, const float* mus
       return fail(h, NMC_EINVAL, msg);
     }
     v[k] = make_float4(a, s, (float)(1.0 / s), gg);
+    sum_a += a;
+    sum_s += s;
   }
   if (!h->d_vox) NMC_CUDA(h, cudaMalloc((void**)&h->d_vox, h->nvox * sizeof(float4)));
   NMC_CUDA(h, cudaMemcpy(h->d_vox, v.data(), h->nvox * sizeof(float4), cudaMemcpyHostToDevice));
+  h->vox_mua = sum_a / (double)h->nvox;
+  h->vox_mus = sum_s / (double)h->nvox;
   h->voxel_mode = true;
   h->adj_ready = false;
   return build_xyz(h);

@@ -10,6 +10,7 @@ import pytest
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 SRC = r"""
 #include "launch_rules.h"
+#include <cstring>
 using namespace nmc;
 static WorkTail one(double n, double mua, double mus) { WorkTail w; w.add(n, mua, mus); return w; }
 extern "C" {
@@ -36,6 +37,22 @@ int layered(unsigned long long n, int nl, const double* q, int ref) {  // 0: the
   const LayeredShape s = layered_shape(w, n, 2432, ref);
   return s.latency ? 0 : s.blocks ? s.blocks : 4;
 }
+int voxel(unsigned long long n, double mua, double mus, int faces) {  // a map of air and this tissue, 2 cm
+  nmc_tissue_params tp;
+  std::memset(&tp, 0, sizeof tp);
+  tp.muav[1] = 1e-4f; tp.musv[1] = 1.f; tp.gv[1] = 1.f;
+  tp.muav[2] = (float)mua; tp.musv[2] = (float)mus; tp.gv[2] = 0.9f;
+  tp.muav[3] = 1e-3f; tp.musv[3] = 100.f; tp.gv[3] = 0.9f;  // not in the map
+  WorkTail w;
+  voxel_add(w, (double)n, tp, false, 6u, 2.0);
+  const VoxelShape s = voxel_shape(w, n, 152, faces, false);
+  return s.block == 256 ? s.per_sm : -s.block;
+}
+int voxel_sweep(int n_sets, double per, const double* mua, const double* mus) {
+  WorkTail w;
+  for (int k = 0; k < n_sets; ++k) w.add(per, mua[k], mus[k]);
+  return voxel_shape(w, (uint64_t)(n_sets * per), 152, false, true).per_sm;
+}
 unsigned lanes(unsigned long long items, unsigned long long warps) { return lat_lanes(items, warps); }
 }
 """
@@ -45,7 +62,8 @@ unsigned lanes(unsigned long long items, unsigned long long warps) { return lat_
 def rules(tmp_path_factory):
     d = tmp_path_factory.mktemp("rules")
     (d / "rules.cpp").write_text(SRC)
-    subprocess.run(["g++", "-O1", "-std=c++17", "-shared", "-fPIC", "-I" + os.path.join(ROOT, "nmc_gb300", "csrc"), str(d / "rules.cpp"),
+    subprocess.run(["g++", "-O1", "-std=c++17", "-shared", "-fPIC", "-I" + os.path.join(ROOT, "nmc_gb300", "csrc"),
+                    "-I" + os.path.join(ROOT, "include"), str(d / "rules.cpp"),
                     "-o", str(d / "rules.so")], check=True)
     lib = C.CDLL(str(d / "rules.so"))
     lib.sub_lat.argtypes = [C.c_double] * 3 + [C.c_int]
@@ -53,6 +71,8 @@ def rules(tmp_path_factory):
     lib.spectrum_lat.argtypes = [C.c_int] + [C.c_void_p] * 3
     lib.field_lat.argtypes = [C.c_double] * 2
     lib.layered.argtypes = [C.c_ulonglong, C.c_int, C.c_void_p, C.c_int]
+    lib.voxel.argtypes = [C.c_ulonglong, C.c_double, C.c_double, C.c_int]
+    lib.voxel_sweep.argtypes = [C.c_int, C.c_double, C.c_void_p, C.c_void_p]
     lib.lanes.argtypes, lib.lanes.restype = [C.c_ulonglong] * 2, C.c_uint
     return lib
 
@@ -139,3 +159,41 @@ def test_layered(rules, name):
         assert rules.layered(n, len(q), a.ctypes.data, 0) == 0
         assert rules.layered(n, len(q), a.ctypes.data, 1) != 0
     assert rules.layered(40_000, len(q), a.ctypes.data, 0) != 0
+
+
+VOXEL = [  # mua, mus, photons, ms at 2, 3, 4 blocks per SM: a cube of one tissue
+    (50, 50, 100_000, (0.109, 0.090, 0.090)), (50, 50, 200_000, (0.191, 0.150, 0.139)), (50, 50, 300_000, (0.278, 0.217, 0.195)),
+    (20, 100, 100_000, (0.258, 0.209, 0.214)), (20, 100, 200_000, (0.425, 0.351, 0.338)), (20, 100, 400_000, (0.804, 0.645, 0.610)),
+    (5, 100, 100_000, (0.758, 0.689, 0.673)), (5, 100, 200_000, (1.177, 1.044, 1.094)), (5, 100, 600_000, (3.082, 2.591, 2.500)),
+    (1, 100, 100_000, (2.997, 3.174, 3.104)), (1, 100, 200_000, (4.663, 4.464, 4.626)), (1, 100, 300_000, (6.356, 5.777, 5.912)),
+    (0.5, 200, 100_000, (13.93, 15.68, 15.52)), (0.5, 200, 300_000, (21.40, 20.37, 23.32)), (0.5, 200, 1_000_000, (48.19, 42.93, 43.50)),
+    (0.2, 100, 100_000, (15.12, 16.07, 15.54)), (0.2, 100, 300_000, (26.18, 24.22, 25.06)),
+]
+
+
+@pytest.mark.parametrize("mua,mus,n,ms", VOXEL)
+def test_voxel(rules, mua, mus, n, ms):
+    assert ms[rules.voxel(n, mua, mus, 0) - 2] <= 1.05 * min(ms)
+    assert rules.voxel(n, mua, mus, 1) == 4
+
+
+@pytest.mark.parametrize("n,block", [(1, 1), (2432, 1), (2433, 2), (12_160, 5)])
+def test_voxel_few_photons(rules, n, block):
+    assert rules.voxel(n, 50.0, 50.0, 0) == rules.voxel(n, 0.5, 200.0, 1) == -block
+
+
+SPECTRA = [  # absorption against the seeded tables', photons, ms at 2, 3, 4 blocks per SM, one-term
+    (1, 300_000, (55.7, 60.8, 59.3)), (1, 1_400_000, (69.2, 76.9, 93.9)), (1, 2_500_000, (120.1, 99.3, 112.7)),
+    (1, 3_500_000, (167.3, 135.5, 140.3)), (1, 7_000_000, (333.4, 269.4, 251.8)), (20, 1_400_000, (7.59, 6.97, 7.16)),
+    (20, 2_500_000, (12.36, 10.48, 10.47)), (20, 5_000_000, (24.7, 19.7, 19.1)), (20, 7_000_000, (34.6, 27.7, 25.5)),
+]
+
+
+@pytest.mark.parametrize("scale,n,ms", SPECTRA)
+def test_voxel_sweep(rules, scale, n, ms):
+    import nmc_cases as cases
+
+    _, tables, _ = cases.skin_vessel_spectral_tables(seed=2024)
+    best = [max(((t.muav[i] * scale + t.musv[i]) / (t.muav[i] * scale), t.muav[i] * scale, t.musv[i]) for i in (2, 3, 4)) for t in tables]
+    mua, mus = (np.array([b[k] for b in best]) for k in (1, 2))
+    assert ms[rules.voxel_sweep(351, n // 351, mua.ctypes.data, mus.ctypes.data) - 2] <= 1.03 * min(ms)
