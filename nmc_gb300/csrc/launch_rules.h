@@ -131,6 +131,11 @@ inline LayeredShape layered_shape(const WorkTail& w, uint64_t photons, uint64_t 
   return {false, photons <= warps * 256 && w.below(1.0e5) ? kLatBlocks : 0};
 }
 
+// The longest side of a run's voxel grid.
+inline double grid_extent(const nmc_run_params& rp) {
+  return std::max({(double)rp.Nx * rp.dx, (double)rp.Ny * rp.dy, (double)rp.Nz * rp.dz});
+}
+
 // n photons in a voxel grid whose longest side is `extent` and whose map holds
 // the tissues of `present` (bit t: tissue t): the longest live in the tissue with
 // the most scatterings per absorption.  A tissue too clear to turn a photon within

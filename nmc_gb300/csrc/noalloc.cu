@@ -160,9 +160,15 @@ extern "C" nmc_status nmc_mcxyz_run_noalloc(const nmc_run_params* rp, const nmc_
     p.trace = nmc::TraceParams{nullptr, nullptr, 0};
     const bool tt = rp->mckernelflag == NMC_SIM_MCXYZ_TT;
     // the launch shape nmc_run takes from the same nmc_ext
-    const int block = ext->block_size > 0 ? ext->block_size : 256;
+    const bool own = ext->block_size <= 0 && ext->blocks_per_sm <= 0;
+    nmc::WorkTail w;
+    nmc::voxel_add(w, (double)n_photons, *tp, tt, mask, nmc::grid_extent(*rp));
+    const nmc::VoxelShape shape =
+        nmc::voxel_shape(w, (n_photons + p.per_fetch - 1) / p.per_fetch, nsm, rp->boundaryflag == 1, false);
+    const int block = own ? shape.block : ext->block_size > 0 ? ext->block_size : 256;
     int per_sm = 0;
     if (nmc::mcxyz_occupancy(tt, false, block, &per_sm) != cudaSuccess) return NMC_EDEVICE;
+    if (own) per_sm = std::min(per_sm, shape.per_sm);
     if (ext->blocks_per_sm > 0) per_sm = std::min(per_sm, (int)ext->blocks_per_sm);
     if (per_sm < 1) return NMC_EDEVICE;
     uint64_t grid = (uint64_t)nsm * per_sm;

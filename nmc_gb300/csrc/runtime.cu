@@ -395,11 +395,6 @@ struct AdjArgs {
 
 nmc_status fold(nmc_handle* h);
 
-// The longest side of the handle's grid.
-double grid_extent(const nmc_run_params& rp) {
-  return std::max({(double)rp.Nx * rp.dx, (double)rp.Ny * rp.dy, (double)rp.Nz * rp.dz});
-}
-
 nmc_status launch(nmc_handle* h, uint64_t first, uint64_t n, nmc_photon_record* d_recs,
                   float4* d_events, uint32_t k_events, const AdjArgs* adj = nullptr) {
   if (!h->prepared) return fail(h, NMC_ESTATE, "nmc_prepare has not been called");
@@ -484,7 +479,7 @@ nmc_status launch(nmc_handle* h, uint64_t first, uint64_t n, nmc_photon_record* 
     if (h->voxel_mode)
       w.add((double)n, h->vox_mua, h->vox_mus);
     else
-      nmc::voxel_add(w, (double)n, h->tp, tt, h->tiss_used, grid_extent(h->rp));
+      nmc::voxel_add(w, (double)n, h->tp, tt, h->tiss_used, nmc::grid_extent(h->rp));
     const nmc::VoxelShape shape =
         nmc::voxel_shape(w, (n + p.per_fetch - 1) / p.per_fetch, h->nsm, h->rp.boundaryflag == 1, false);
     block = own ? shape.block : h->ext.block_size > 0 ? h->ext.block_size : 256;
@@ -1394,7 +1389,7 @@ nmc_status nmc_run_sweep_tissues(nmc_handle* h, const nmc_tissue_params* tables,
   const bool own = h->ext.block_size <= 0 && h->ext.blocks_per_sm <= 0;
   nmc::WorkTail w;
   for (int s = 0; s < n_sets; ++s)
-    nmc::voxel_add(w, (double)photons[s], tables[s], tt, h->tiss_used, grid_extent(h->rp));
+    nmc::voxel_add(w, (double)photons[s], tables[s], tt, h->tiss_used, nmc::grid_extent(h->rp));
   const nmc::VoxelShape shape =
       nmc::voxel_shape(w, (p.n + p.per_fetch - 1) / p.per_fetch, h->nsm, h->rp.boundaryflag == 1, true);
   const int block = own ? shape.block : h->ext.block_size > 0 ? h->ext.block_size : 256;
