@@ -55,6 +55,7 @@
 #include <vector>
 
 #include "engine.h"
+#include "speckle_math.cuh"
 #include "nmc_abi.h"
 
 namespace nmc {
@@ -641,109 +642,13 @@ __global__ void cgemm_kernel(const float2* __restrict__ A, const float2* __restr
 //
 // The GPU's FP64 pipe issues 2 lanes per clock per SM, 1/64 of the FP32 rate,
 // and a record took about 600 of its instructions: 3.84 ms for 4.2e6 records.
-// Here each function is evaluated in pairs of floats (hi + lo, about 44 bits:
-// two-sum and fused two-product, Dekker 1971 and Knuth) and rounded once, so
-// the results keep the accuracy of the double functions; arguments outside the
-// range the pair arithmetic covers take the double expressions.  A 256 x 256
-// map with 64 records per pixel went from 5.15 ms to 1.37 ms a call, most of
-// it now the copies of 125 MB; the relative error against 64 bits is 7.2e-8
-// before and after (the float sums over the records dominate it).
+// Here each function is evaluated in pairs of floats and rounded once
+// (speckle_math.cuh: within 0.51 units in the last place, where a double
+// function's rounded result is within 0.5).  A 256 x 256 map with 64 records per
+// pixel went from 5.15 ms to 1.37 ms a call, most of it now the copies of 125 MB;
+// the relative error against 64 bits is 7.2e-8 before and after (the float sums
+// over the records dominate it).
 __device__ __forceinline__ float keep_finite(float v) { return isfinite(v) ? v : 0.0f; }
-
-struct FF {
-  float h, l;
-};
-__device__ __forceinline__ FF two_sum(float a, float b) {
-  const float s = __fadd_rn(a, b), t = __fsub_rn(s, a);
-  return {s, __fadd_rn(__fsub_rn(a, __fsub_rn(s, t)), __fsub_rn(b, t))};
-}
-__device__ __forceinline__ FF fast_two_sum(float a, float b) {  // |a| >= |b|
-  const float s = __fadd_rn(a, b);
-  return {s, __fsub_rn(b, __fsub_rn(s, a))};
-}
-__device__ __forceinline__ FF two_prod(float a, float b) {
-  const float p = __fmul_rn(a, b);
-  return {p, __fmaf_rn(a, b, -p)};
-}
-
-// pi as three floats: hi + mid + lo
-constexpr float kPi1 = 3.14159274f, kPi2 = -8.74227766e-8f, kPi3 = -3.43e-15f;
-
-// x - k unit pi for a small integer k (unit = 2 or 1/2): the product with the
-// leading float is exact as a pair, and x lies within a factor of two of it
-__device__ __forceinline__ FF reduce_pi(float x, float k, float unit) {
-  const FF p = two_prod(k, unit * kPi1);
-  const FF r = two_sum(__fsub_rn(x, p.h), -p.l);
-  const FF q = two_prod(k, unit * kPi2);
-  const FF t = two_sum(r.h, -q.h);
-  return fast_two_sum(t.h, t.l + (r.l - q.l) - k * (unit * kPi3));
-}
-
-__device__ __noinline__ float wrap_slow(float a) { return (float)atan2(sin((double)a), cos((double)a)); }
-
-// atan2(sin a, cos a): a - 2 pi k in (-pi, pi]
-__device__ __forceinline__ float wrap_ref(float a) {
-  const float m = fabsf(a);
-  if (m < kPi1) return a;             // the floats below kPi1 are below pi
-  if (!(m < 4096.f)) return wrap_slow(a);
-  FF r = reduce_pi(a, rintf(a * (0.5f / kPi1)), 2.f);
-  const float s = copysignf(1.f, r.h);
-  if (fabsf(r.h) > kPi1 || (fabsf(r.h) == kPi1 && s * r.l > kPi2)) {  // beyond +-pi: one turn back
-    const FF t = two_sum(r.h, -s * (2.f * kPi1));
-    r = fast_two_sum(t.h, t.l + (r.l - s * (2.f * kPi2)));
-  }
-  return r.h;
-}
-
-// sin x for |x| <= 4, by reduction to [-pi/4, pi/4] and the Taylor series, its
-// leading terms as pairs
-__device__ __forceinline__ float sin_ref(float x) {
-  const float k = rintf(x * (2.f / kPi1));
-  const FF y = k == 0.f ? FF{x, 0.f} : reduce_pi(x, k, 0.5f);
-  const FF z = two_prod(y.h, y.h);
-  const float zl = fmaf(2.f * y.h, y.l, z.l);
-  const int q = (int)k & 3;
-  float v;
-  if (q & 1) {
-    const float c = fmaf(fmaf(fmaf(-2.75573192e-7f, z.h, 2.48015873e-5f), z.h, -1.38888889e-3f), z.h, 4.16666667e-2f);
-    const FF t = fast_two_sum(1.f, -0.5f * z.h);
-    v = t.h + (t.l + fmaf(c * z.h, z.h, -0.5f * zl));
-  } else {
-    const float c = fmaf(fmaf(fmaf(2.75573192e-6f, z.h, -1.98412698e-4f), z.h, 8.33333333e-3f), z.h, -1.66666667e-1f);
-    v = y.h + fmaf(c * z.h, y.h, y.l);
-  }
-  return q & 2 ? -v : v;
-}
-
-// e^a for a <= 0
-__device__ __forceinline__ float exp_ref(float a) {
-  if (!(a > -87.f)) return (float)exp((double)a);  // NaN, or below the normal floats
-  constexpr float kLn1 = 0.693147182f, kLn2 = -1.90465421e-9f;  // ln 2 as two floats
-  const float n = rintf(a * 1.44269504f);
-  const FF p = two_prod(n, kLn1);
-  const FF r = two_sum(__fsub_rn(a, p.h), -fmaf(n, kLn2, p.l));
-  const float c = fmaf(fmaf(fmaf(fmaf(fmaf(1.98412698e-4f, r.h, 1.38888889e-3f), r.h, 8.33333333e-3f), r.h, 4.16666667e-2f),
-                            r.h, 1.66666667e-1f), r.h, 0.5f);
-  const FF t = fast_two_sum(1.f, r.h);
-  return (t.h + (t.l + fmaf(c * r.h, r.h, r.l))) * __int_as_float((127 + (int)n) << 23);
-}
-
-__device__ __noinline__ float interfere_slow(float a, float c, float interf, float env) {
-  const double two = 2.0;  // MC_TWO (definitions.h:60)
-  return (float)(((double)(a + c) + two * sqrt((double)(a * c)) * interf * env) / 4.0f);
-}
-
-// (a + c + 2 sqrt(a c) interf env) / 4
-__device__ __forceinline__ float interfere(float a, float c, float interf, float env) {
-  const float p = a * c;
-  if (!(p >= 0.f && fabsf(a) < 1e15f && fabsf(c) < 1e15f)) return interfere_slow(a, c, interf, env);
-  const float s = __fsqrt_rn(p);
-  const float sl = s > 0.f ? __fdividef(__fmaf_rn(-s, s, p), 2.f * s) : 0.f;
-  const FF w = two_prod(interf, env);
-  const FF u = two_prod(s, w.h);
-  const FF t = two_sum(a + c, 2.f * u.h);
-  return 0.25f * (t.h + (t.l + 2.f * (u.l + fmaf(s, w.l, sl * w.h))));
-}
 
 __global__ void __launch_bounds__(64) speckle_mutual_kernel(int npix, const float* __restrict__ maps,
                                                             const nmc_speckle* __restrict__ rec,
