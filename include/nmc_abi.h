@@ -608,7 +608,9 @@ static_assert(sizeof(nmc_tune_result) == 1004, "nmc_tune_result layout");
  * flight per SM; photons a thread takes from the work queue at a time; for
  * mcsub, tallies privatised in shared memory or not), keeps the fastest in
  * the handle's nmc_ext (block_size, blocks_per_sm, photons_per_fetch, flags) and
- * clears the tallies.  Results do not depend on the configuration: every
+ * clears the tallies.  A kept block_size or blocks_per_sm stands for all later
+ * runs of the handle, whatever their size, where 0 lets the library choose the
+ * shape for each run: tune a handle at the size it is to run.  Results do not depend on the configuration: every
  * photon's stream is a function of its id only.  No reference counterpart
  * (the reference dispatches 1e4 threads in threadgroups of the pipeline's
  * maximum, MetalMC.m:485-495). */

@@ -202,7 +202,7 @@ __device__ __forceinline__ void perp_of(float ux, float uy, float uz, float& px,
   }
 }
 
-// LAT: the latency variant (engine.h)
+// LAT: the latency variant (launch_rules.h)
 template <bool FAST, bool LAT>
 __global__ void __launch_bounds__(kLatBlock, LAT ? kLatBlocks : 4) efield_kernel(const EfParams P) {
   using M = Math<FAST>;

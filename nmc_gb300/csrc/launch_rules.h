@@ -43,7 +43,7 @@ inline unsigned int lat_lanes(uint64_t items, uint64_t warps) {
 }
 
 // The semi-infinite kernel's latency variant.  Its private F(r,z) can leave
-// room for one block per SM only (bins 118 to 158): the variant then has 8
+// room for one block per SM only (bins 119 to 158): the variant then has 8
 // warps per SM where the other kernel has 16, and pays up to a smaller ratio.
 // 128 bins, variant against the other, at photons of (mua, mus): (1, 100) 1e4
 // 0.59 / 0.96 ms, 7e4 0.89 / 0.98, 1e5 1.10 / 1.00, 3e5 2.54 / 1.94; (10, 100)

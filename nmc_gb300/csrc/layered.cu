@@ -49,8 +49,8 @@
 // a carry of the A(z) sum) behind one test, and goes on to the interaction
 // after a crossing.  Three-layer skin, 4e6 photons of 1520 interactions:
 // 69.4 -> 53.6 ms, 10.3 -> 8.0 warp instructions per interaction at 21.0 ->
-// 22.9 active lanes (1e6 photons: 26.9 -> 21 ms, 10 ms of it the longest
-// photon).
+// 22.9 active lanes (1e6 photons: 26.9 -> 20 ms, of which the longest photon
+// alone takes 10).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -106,7 +106,7 @@ struct LayParams {
   int iso;            // isotropic scattering (the reference's mcsub sampling)
 };
 
-// LAT: the latency variant (engine.h)
+// LAT: the latency variant (launch_rules.h)
 template <bool FAST, bool ADJ, bool REF, bool LAT>
 __global__ void __launch_bounds__(kLatBlock, LAT ? kLatBlocks : 4) layered_kernel(const LayParams P) {
   using M = Math<FAST>;

@@ -383,8 +383,9 @@ size_t mcsub_smem_bytes(int bins) {
   return 2 * (nF + nJ) * sizeof(uint32_t);
 }
 
-// Shared-memory privatisation while the tally fits next to a second block
-// (BINS <= 160); larger grids deposit straight into the global u64 tally.
+// Shared-memory privatisation while the tally fits a block (BINS <= 158; two
+// blocks per SM up to 118, one beyond); larger grids deposit straight into the
+// global u64 tally.
 static bool smem_fits(int bins) { return mcsub_smem_bytes(bins) <= 200 * 1024; }
 
 static cudaError_t prepare(const SubParams& p, bool trace, const void** f, size_t* sh) {

@@ -6,12 +6,12 @@
 // (NMC-samples/example3.ipynb cell 5).  Here every set's photon budget is a
 // slice of one global photon index space: threads take photon indices from
 // a warp-aggregated counter (work stealing across sets), find the photon's
-// set by binary search over the budgets' prefix sums, and read that set's
-// optical constants through the read-only cache.  The host lays the sets
-// out in decreasing order of estimated cost per photon, so the photons that
-// live longest start first.  Uneven budgets therefore
-// cost nothing extra: the GPU stays full until the last photon of the last
-// set, and there is one tail for the whole sweep instead of one per set.
+// set by binary search over the budgets' prefix sums, and load that set's
+// optical constants.  The host lays the sets out in decreasing order of
+// estimated cost per photon, so the photons that live longest start first.
+// Uneven budgets therefore cost nothing extra: the GPU stays full until the
+// last photon of the last set, and there is one tail for the whole sweep
+// instead of one per set.
 // Per-set totals are u64 fixed point in shared memory, folded into global
 // memory once per block; the escaping flux J(r) of each set goes straight to
 // global u64 atomics (one deposit per escaping photon).
@@ -24,7 +24,8 @@
 // blocks (and 85.6 ms with the constants in registers squeezed to 4 blocks);
 // 3.5e6 photons, where fewer resident photons also shorten the tail, 37.6
 // against 53.8 ms.  Sweeps whose tail outweighs their work take the latency
-// variant (99 registers, thin warps): the 3.5e6 photons 28.6 ms.
+// variant (99 registers, thin warps): the 3.5e6 photons 28.6 ms.  Large one-term
+// sweeps run 4 blocks (64 registers, no spills): launch_rules.h.
 #include <cuda_runtime.h>
 
 #include "engine.h"
